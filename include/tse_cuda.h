@@ -143,9 +143,12 @@ int32_t tse_compute_P(const TseGrid *grid, const TsePressureArgs *args,
  * red-black SOR sweeps on an FP32 correction, which is added to the FP64
  * iterate every `cycle` iterations and at convergence.  Same arguments,
  * convergence test, dt control and results as the FP64 entry points;
- * agreement with them is to the solver tolerance, not bit for bit.  These
- * calls synchronise the stream once per correction cycle (they read the
- * sweep kernel's event record) and return when the solve is done.
+ * agreement with them is to the solver tolerance, not bit for bit.  A grid
+ * whose FP32 state fits on the chip (up to about 0.9M cells on a B200) solves
+ * in one launch, cycles included, unless a staged variant is named in
+ * `opts`; for larger grids the calls synchronise the stream once per
+ * correction cycle (they read the sweep kernel's event record).  Not for a
+ * stream that is being captured.
  * Workspace: TSE_WS_PRESSURE_DC / TSE_WS_TRANSPORT_DC. */
 typedef struct TseDcOptions {
     int32_t cycle;            /* in: iterations per correction cycle, <= 0: 256 */
@@ -154,7 +157,8 @@ typedef struct TseDcOptions {
     int32_t timing;           /* in: 1 = time the sweep-kernel launches (CUDA
                                  events on the call's stream; the global timer
                                  inside the device-driven loop's graph) */
-    int32_t sweep_launches;   /* out (timing): sweep-kernel launches */
+    int32_t sweep_launches;   /* out (timing): sweep-kernel launches (a
+                                 resident solve is one, residuals included) */
     int64_t sweep_iterations; /* out (timing): red+black iterations they ran */
     double sweep_ms;          /* out (timing): their summed event time */
     int32_t host_loop;        /* in, batched fused form only: 0 (default) the
@@ -170,7 +174,11 @@ typedef struct TseDcOptions {
     int32_t chunk;            /* in/out, single-model forms: the staged sweep's
                                  chunk of cells (256, 512, 1024; else 512) --
                                  on return the variant that ran, 0 for the
-                                 plain-load sweep (no stages fit) */
+                                 resident solve and for the plain-load sweep
+                                 (no stages fit).  chunk, ring and pipes all 0:
+                                 the library's choice, the resident solve
+                                 where it fits; any of them set: the staged
+                                 sweep */
     int32_t ring;             /* in/out: stages a pipeline (2..4; else as many
                                  as fit, up to 4) */
     int32_t pipes;            /* in/out: pipelines a block (1: two blocks per

@@ -31,7 +31,9 @@ import torch
 CHUNKS = (256, 512, 1024)
 RINGS = (2, 3, 4)
 PIPES = (2, 1)
-VARIANTS = tuple((c, r, p) for c in CHUNKS for p in PIPES for r in RINGS)
+# (0, 0, 0): the library's choice -- a grid that fits on the chip solves
+# resident, without a staged sweep; naming a variant asks for the staged one
+VARIANTS = ((0, 0, 0),) + tuple((c, r, p) for c in CHUNKS for p in PIPES for r in RINGS)
 
 _chosen = {}
 
@@ -88,7 +90,7 @@ def tune_sweep(sim, iters=64, repeats=3, variants=VARIANTS, cache=True):
             failed.append({"variant": tuple(v), "error": str(e)})
             ran = None
         sim.S["P"].copy_(P0)
-        if ran is None or ran[0] == 0 or ran in seen:
+        if ran is None or ran in seen or (ran[0] == 0 and any(v)):
             continue   # the plain-load sweep ran, or a variant already timed
         seen.add(ran)
         trials.append({"chunk": ran[0], "ring": ran[1], "pipes": ran[2],
@@ -97,7 +99,7 @@ def tune_sweep(sim, iters=64, repeats=3, variants=VARIANTS, cache=True):
     if not trials:
         M.sweep_variant = (0, 0, 0)
         return {"variant": (0, 0, 0), "trials": [], "failed": failed,
-                "note": "no staged variant fits this grid"}
+                "note": "no variant ran"}
     best = min(trials, key=lambda t: t["us_per_iteration"])
     rec = {"variant": (best["chunk"], best["ring"], best["pipes"]),
            "us_per_iteration": best["us_per_iteration"], "iters": iters, "trials": trials}

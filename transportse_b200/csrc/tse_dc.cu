@@ -33,6 +33,7 @@
 //
 // Compiled with FMA contraction (no bit-exactness is claimed for this form).
 #include "tse_dc.cuh"
+#include "tse_dc_resident.cuh"
 
 namespace tse {
 
@@ -566,6 +567,10 @@ size_t dc_extra_bytes(const Layout& L) {
            align256(sizeof(DcState)) + 256 + 512;
 }
 
+size_t dc_resident_bytes(const Layout& L) {
+    return L.Nc <= kDcResMaxNc ? dc_res_bytes(L) : 0;
+}
+
 static int sweep_blocks(long long Nc, int cap) {
     static int cached_dev = -1, cached_per_sm = 0, cached_sms = 0;
     int dev = 0;
@@ -662,6 +667,13 @@ static int run_dc(SolveSetup<Form>& S, double dt, double inc_it, double max_dt, 
     c.stop_on_first = stop_on_first;
     c.cycle = cycle > 0 ? cycle : 256;
     c.sor = (float)sor;
+    const bool timing = opts && opts->timing;
+    // a grid that fits on the chip, and no staged variant asked for
+    if (!opts || (opts->chunk == 0 && opts->ring == 0 && opts->pipes == 0)) {
+        const int rc = run_dc_resident(S, c, dt, cap, first_parts, X_out, d_status, timing ? opts : nullptr,
+                                       stream);
+        if (rc != 1) return rc;
+    }
     const long long dlen = dc_delta_len(S.L, S.Ncal);
     float* dbase = c.D[0] - dc_margin(S.L);
     // the margins must read as 0 (kernels rewrite the interior only)
@@ -702,7 +714,6 @@ static int run_dc(SolveSetup<Form>& S, double dt, double inc_it, double max_dt, 
         dc_scale_kernel<<<gcells, kBlock, 0, stream>>>(S.F, c);
         if (cudaGetLastError() != cudaSuccess) return TSE_ERR_LAUNCH;
     }
-    const bool timing = opts && opts->timing;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     if (timing) {
         opts->sweep_launches = 0;
