@@ -87,10 +87,11 @@ typedef struct TsePressureArgs {
     double dt_P, SOR, inc_it, max_dt, min_dt, P_conv;
     int32_t max_it;
     int32_t sweep;    /* FP64 solves' sweep kernel for this call (no counterpart
-                         in the reference): 0 the bulk-copy staged kernel
-                         wherever its stages fit, else plain loads (default);
-                         1 plain loads.  Same cell values either way.  The
-                         mixed-precision forms ignore it. */
+                         in the reference): 0 (default) the resident kernel
+                         where the grid's state fits on the chip, else as 2;
+                         1 plain loads; 2 the bulk-copy staged kernel wherever
+                         its stages fit, else plain loads.  Same cell values
+                         either way.  The mixed-precision forms ignore it. */
 } TsePressureArgs;
 
 /* Species transport arguments, compute_C(C, D_fx, D_fy, D_fz, phi, rho_f,

@@ -127,3 +127,51 @@ def test_transport_solves_equal_the_staged_form(shape, omega, cuda_device):
         (r, ran, _), (s, _, _) = _both(cfg, cuda_device, call)
         assert ran == (0, 0, 0)
         _same(r, s)
+
+
+# FP64: one block (at most 480 groups of two cells), clusters, the whole GPU, too large
+EXACT = [((12, 10, 16), True), ((11, 11, 16), True), ((24, 24, 24), True), ((33, 17, 21), True),
+         ((48, 48, 48), True), ((60, 52, 60), True), ((80, 80, 80), False), ((1, 1, 1), True),
+         ((1, 1, 900), True), ((1, 60, 30), True), ((200, 1, 3), True), ((5, 7, 2), True)]
+
+
+@pytest.mark.parametrize("shape,resident", EXACT)
+def test_exact_solves_equal_the_streaming_kernels(shape, resident, cuda_device):
+    """FP64 pressure and species solves (x and z buoyancy, omega < 1, the
+    IMBLFLO term), resident, staged and with plain loads: the same bits; and
+    dt halvings, a stop at min_dt and a NaN."""
+    import ctypes as ct
+    from transportse_b200 import _native as N
+    cfg, rng, args, P, BP, WP = _case(shape, 21)
+    cfg.lf_l[:] = rng.uniform(0, 1, shape)
+    cfg.lf_t[:] = rng.uniform(0, 0.3, shape)
+    cfg.C_IMBLFLO = True
+    C = rng.uniform(0, 1, shape)
+    D = 1e-6 * rng.uniform(0.5, 1.5, shape)
+    B = (rng.uniform(size=shape) < 0.1).astype(float)
+    W = numpy.where(rng.uniform(size=shape) < 0.2, 1e-5, 0.0)
+    e = rng.uniform(-1e-6, 1e-6, shape)
+    q = [rng.uniform(-1e-4, 1e-4, shape) for _ in range(3)]
+    one, z = numpy.ones(shape), numpy.zeros(shape)
+    bad = P.copy()
+    bad.reshape(-1)[-1] = numpy.nan
+    m = model_for(cfg, cuda_device)
+    # the workspace carries the exchange records just where the form may run
+    plain = N.lib().tse_workspace_bytes(ct.byref(m.grid), N.TSE_WS_PRESSURE)
+    assert m.ws_bytes >= plain
+    nk = NumpyKernels(m)
+    out = []
+    for mode in (0, 2, 1):
+        m.sweep = mode
+        got = []
+        for p0, max_it, min_dt in ((P, 20000, 1e-8), (P, 40, 1.0), (P, 7, 400.0), (bad, 12, 1000.0)):
+            r = nk.compute_P(p0.copy(), *args, z, z, z, 3600.0, BP, WP, SOR=1.7, max_it=max_it, inc_it=1.25,
+                             max_dt=1e5, min_dt=min_dt, P_conv=1e-10)
+            s = m.last_status
+            got += [*r, s.num_sub_it, s.halvings, s.n_events]
+        for omega in (1.0, 0.5, 0.0):
+            got += [*nk.compute_C(C.copy(), D, D, D, args[3], args[2], *q, 600.0, B, W, one, e, omega=omega,
+                                  SOR=1.1, max_it=100, inc_it=1.05, max_dt=1e5, min_dt=1e-8, C_conv=1e-11)]
+        out.append(got)
+    _same(out[0], out[1])
+    _same(out[0], out[2])

@@ -365,7 +365,8 @@ static int run_dc_resident(SolveSetup<Form>& S, DcCtl& c, double dt, int cap, in
         cluster = form == 0;
         int maxb = cluster ? kDcResCluster : sms < kResMaxBlocks ? sms : kResMaxBlocks;
         if (cap > 0 && maxb > cap) maxb = cap;
-        if (!res_plan(S.L, kDcResVals, maxb, kDcResGroups2, room, dc_res_smem, dc_res_threads, P)) continue;
+        if (!res_plan(S.L, kDcResVals, maxb, kDcResGroups2, room, dc_res_smem, dc_res_threads, true, P))
+            continue;
         if (P.nb == 1) cluster = false;
         threads = dc_res_threads(P);
         const bool one = threads == 512;

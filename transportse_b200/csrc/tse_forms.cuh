@@ -72,6 +72,29 @@ struct PressureForm {
         return n;
     }
     static constexpr int kSolution = PA_P;
+    static constexpr int kDen = PA_DEN, kRhs = PA_RPN;
+    // The resident solve's arrays of a group, in a fixed order for either
+    // switch (x buoyancy, z buoyancy); an odd number, so that consecutive
+    // groups' loads fall into different shared-memory banks
+    static constexpr int kCoef = PA_DEN + 1;
+    template <bool G1, bool G2>
+    static __host__ __device__ constexpr int res_arrays() { return 9 + 2 * G1 + 2 * G2; }
+    template <bool G1, bool G2>
+    static __host__ __device__ constexpr int res_slot(int k) {
+        return k < PA_AB ? k
+             : k < PA_IJ ? (G1 ? k : -1)
+             : k < PA_RPN ? (G2 ? k - 2 * !G1 : -1)
+                          : k - 2 * !G1 - 2 * !G2;
+    }
+    bool res_g1() const { return xgrav != 0; }
+    bool res_g2() const { return zgrav != 0; }
+    template <bool G1, bool G2>
+    __device__ __forceinline__ PressureForm res_form() const {
+        PressureForm f = *this;
+        f.xgrav = G1;
+        f.zgrav = G2;
+        return f;
+    }
     static constexpr int kArrays = PA_COUNT;
     __device__ __forceinline__ double den(int col, long long m) const {
         return arr[col][PA_DEN * Ncal + m];
@@ -152,6 +175,28 @@ struct TransportForm {
         return n;
     }
     static constexpr int kSolution = TA_X;
+    static constexpr int kDen = TA_DEN, kRhs = TA_RXN;
+    // as PressureForm's; the switches are useY and useEX
+    static constexpr int kCoef = TA_DEN + 1;
+    template <bool G1, bool G2>
+    static __host__ __device__ constexpr int res_arrays() { return (9 + G1 + G2) | 1; }
+    template <bool G1, bool G2>
+    static __host__ __device__ constexpr int res_slot(int k) {
+        return k < TA_Y ? k
+             : k == TA_Y ? (G1 ? k : -1)
+             : k < TA_EX ? k - !G1
+             : k == TA_EX ? (G2 ? k - !G1 : -1)
+                          : k - !G1 - !G2;
+    }
+    bool res_g1() const { return useY != 0; }
+    bool res_g2() const { return useEX != 0; }
+    template <bool G1, bool G2>
+    __device__ __forceinline__ TransportForm res_form() const {
+        TransportForm f = *this;
+        f.useY = G1;
+        f.useEX = G2;
+        return f;
+    }
     static constexpr int kArrays = TA_COUNT;
     __device__ __forceinline__ double den(int col, long long m) const {
         return arr[col][TA_DEN * Ncal + m];

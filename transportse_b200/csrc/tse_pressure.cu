@@ -15,6 +15,7 @@
 #include "tse_dc.cuh"
 #include "tse_forms.cuh"
 #include "tse_rbsolve.cuh"
+#include "tse_rbsolve_res.cuh"
 #include "tse_rbsolve_tma.cuh"
 
 namespace tse {
@@ -200,6 +201,9 @@ size_t pressure_ws_bytes(const Layout& L, long long* Ncal_out) {
     return b;
 }
 
+// exchange memory of the resident FP64 solves, after the arrays
+size_t fp64_resident_bytes(const Layout& L) { return x_res_bytes(L); }
+
 // Carve the workspace and launch the assembly (shared by the exact and the
 // defect-correction pressure solves).  The bytes after the exact form's
 // arrays are returned in `tail` for the caller's own use.
@@ -309,6 +313,10 @@ extern "C" int32_t tse_compute_P(const TseGrid* grid, const TsePressureArgs* arg
     ctl.partials = S.partials;
     ctl.bar = S.bar;
     ctl.status = d_status;
+    if (args->sweep != 1 && args->sweep != 2) {
+        rc = launch_rb_resident(S.F, ctl, S.tail, S.tail_bytes, args->P, stream);
+        if (rc != 1) return rc;
+    }
     rc = launch_rb_solve_tma(S.F, ctl, stream);
     if (rc == 1) rc = launch_rb_solve(S.F, ctl, stream);
     if (rc != TSE_OK) return rc;

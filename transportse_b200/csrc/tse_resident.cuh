@@ -53,11 +53,11 @@ constexpr int kResMaxThreads = 512;
 // A plan for the layout (vals cells a group) on at most maxb blocks, at most
 // max_groups groups per colour and tile, dynamic shared memory smem(plan) <=
 // smem_max.  The plan with the smallest largest tile, edges weighed against
-// cells; one block when everything fits in it, since a half-sweep of one
-// block exchanges nothing.
+// cells; one block when one_first and everything fits in it, since a
+// half-sweep of one block exchanges nothing.
 template <class SmemFn, class ThreadsFn>
 inline bool res_plan(const Layout& L, int vals, int maxb, int max_groups, int smem_max, SmemFn smem,
-                     ThreadsFn threads, ResPlan& best) {
+                     ThreadsFn threads, bool one_first, ResPlan& best) {
     double best_cost = 0.0;
     bool found = false;
     const int Hg = (L.H + vals - 1) / vals;
@@ -86,7 +86,7 @@ inline bool res_plan(const Layout& L, int vals, int maxb, int max_groups, int sm
             if (P.smem > smem_max) continue;
             // a second round of polling costs about what 250 groups' sweep does
             const double cost =
-                P.nb == 1 ? -1.0 : (double)groups + 0.5 * P.halo + (P.halo > threads(P) ? 250.0 : 0.0);
+                P.nb == 1 && one_first ? -1.0 : (double)groups + 0.5 * P.halo + (P.halo > threads(P) ? 250.0 : 0.0);
             if (!found || cost < best_cost) {
                 best = P;
                 best_cost = cost;

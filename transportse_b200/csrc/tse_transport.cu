@@ -12,6 +12,7 @@
 #include "tse_dc.cuh"
 #include "tse_forms.cuh"
 #include "tse_rbsolve.cuh"
+#include "tse_rbsolve_res.cuh"
 #include "tse_rbsolve_tma.cuh"
 
 namespace tse {
@@ -663,6 +664,10 @@ static int run_transport(const TseGrid* grid, const Args* a, double* X, TseSolve
     ctl.partials = w.partials;
     ctl.bar = w.bar;
     ctl.status = d_status;
+    if (a->sweep != 1 && a->sweep != 2) {
+        rc = launch_rb_resident(F, ctl, S.tail, S.tail_bytes, X, stream);
+        if (rc != 1) return rc;
+    }
     rc = launch_rb_solve_tma(F, ctl, stream);
     if (rc == 1) rc = launch_rb_solve(F, ctl, stream);
     if (rc != TSE_OK) return rc;

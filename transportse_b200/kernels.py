@@ -74,8 +74,9 @@ class Model:
         self.T_IMBLFLO = False
         self.last_status = None
         self.launches = 0
-        # FP64 solves' sweep kernel (args.sweep): 0 the bulk-copy staged
-        # kernel where its stages fit, 1 plain loads; same cell values
+        # FP64 solves' sweep kernel (args.sweep): 0 resident where the grid
+        # fits on the chip, else staged; 1 plain loads; 2 the bulk-copy staged
+        # kernel where its stages fit; same cell values
         self.sweep = 0
         # mixed-precision solves: the staged FP32 sweep's variant (chunk
         # cells, ring stages, pipelines per block; 0 = the library's
