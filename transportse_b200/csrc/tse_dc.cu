@@ -45,9 +45,6 @@ constexpr int kSweepMinBlocks = TSE_SWEEP_MINB;
 #define TSE_SWEEP_BLOCK 256
 #endif
 constexpr int kSweepBlock = TSE_SWEEP_BLOCK;
-#ifndef TSE_TMA_PREFETCH
-#define TSE_TMA_PREFETCH 1   // 1: a phase's own parts are copied before its grid barrier
-#endif
 
 // Pipelines of the staged sweep: each has its own producer warp, its own ring
 // of stages and its own consumer group, and takes every PIPES-th chunk of the
@@ -60,7 +57,7 @@ constexpr int kDcPipes = 2;
 constexpr int kDcMaxRing = 4;
 template <int PIPES>
 struct DcLayout {
-    static constexpr int kThreads = kTmaConsumers + 32 * PIPES;
+    static constexpr int kThreads = kTmaConsumers + 32 * PIPES + 64;   // consumers, producers, reporter, gatekeeper
     static constexpr int kMinBlocks = PIPES == 1 ? 2 : 1;
     static constexpr int kGroupsPerPipe = (kTmaConsumers / kTmaGroup) / PIPES;
     static_assert((kTmaConsumers / kTmaGroup) % PIPES == 0, "every pipeline has its own consumer groups");
@@ -276,6 +273,46 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) dc_sweep_kernel(
 
 // ------------------------------------------------ FP32 sweeps, bulk-copy staged
 // (the staging pieces are in tse_dc.cuh)
+//
+// Colour phases are not separated by a device-wide barrier: a phase's first
+// rounds begin while the phase before ends (sweep_head), so the copy pipelines
+// run on from one phase into the next; only iterations that check the
+// convergence end in a barrier.  A report costs the block no time of its own:
+// the consumers arrive on a barrier of the block, a reporter warp waits there
+// and makes their stores visible to the GPU, and a gatekeeper warp waits for
+// the other blocks and opens the next rounds to the producers.  Every one of
+// these steps on a consumer's or a producer's path made the sweep slower than
+// the device-wide barrier did (consumers' fences 2.5 times, the producers'
+// polls 1.5 times, the producers' proxy fences 1.2 times).  Bound: DRAM, 29
+// bytes an update, and below about 3M cells the producers' issue rate (7 copies
+// a chunk, 100 ns each).  Barrier after every phase and now, us per iteration
+// of the sweep alone (B200, both on one box, twice): 128^3 15.2 -> 14.6, 192 x
+// 192 x 128 26.2 -> 23.3, 256 x 256 x 128 42.0-42.8 -> 39.7-42.3 (0.94 of the
+// measured HBM rate at best), 320 x 320 x 160 88.3 -> 82.6-83.5.
+// seg_wait: a report's count has reached `target` (acquire); bounded.
+__device__ __forceinline__ bool seg_wait(const unsigned* count, unsigned target, GridBarrier* bar,
+                                         volatile int* err) {
+    if ((int)(ld_acquire_u32(count) - target) >= 0) return true;
+    const uint64_t t0 = globaltimer();
+    unsigned spins = 0;
+    while ((int)(ld_acquire_u32(count) - target) < 0) {
+        if ((++spins & 63u) == 0u &&
+            (*err || *(volatile int*)&bar->error || globaltimer() - t0 > kBarrierTimeoutNs)) {
+            *err = 1;
+            atomicExch(&bar->error, 1);
+            return false;
+        }
+        __nanosleep(32);
+    }
+    return true;
+}
+
+// A consumer warp has finished its chunks of one report.
+__device__ __forceinline__ void seg_arrive(uint64_t* bar) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+}
+
 template <int RING, int PIPES, int CHUNK>
 __global__ void __launch_bounds__(DcLayout<PIPES>::kThreads, DcLayout<PIPES>::kMinBlocks)
     dc_sweep_tma_kernel(DcCtl c, TmaStage T) {
@@ -287,11 +324,14 @@ __global__ void __launch_bounds__(DcLayout<PIPES>::kThreads, DcLayout<PIPES>::kM
     __shared__ __align__(8) uint64_t full[RING * PIPES];
     __shared__ __align__(8) uint64_t empty[RING * PIPES];
     __shared__ double sh[kThreads / 32];
+    __shared__ __align__(8) uint64_t seg_bar[kSegs], gate[kSegs];
     __shared__ int s_err;
     const unsigned nb = gridDim.x, b = blockIdx.x;
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
-    const bool producer = warp >= kTmaConsumers / 32;
+    const bool reporter = warp == kTmaConsumers / 32 + kPipes;
+    const bool gatekeeper = warp == kTmaConsumers / 32 + kPipes + 1;
+    const bool producer = !reporter && !gatekeeper && warp >= kTmaConsumers / 32;
     const int group = tid / kTmaGroup;                  // consumers: 0 or 1
     const int gt = tid & (kTmaGroup - 1);               // thread within its group
     // this thread's pipeline (producer warp + its ring of stages +
@@ -307,8 +347,22 @@ __global__ void __launch_bounds__(DcLayout<PIPES>::kThreads, DcLayout<PIPES>::kM
     const long long mine = nch > (long long)b ? (nch - 1 - b) / nb + 1 : 0;   // chunks of this block
     // this pipeline's chunks of a phase: i = pipe, pipe + kPipes, ...
     const long long pmine = mine > pipe ? (mine - 1 - pipe) / kPipes + 1 : 0;
-    unsigned* bar_count = c.prog;   // count_sync's counter, zeroed before the launch
-    unsigned bars = 0;              // device-wide barriers passed in this launch
+    unsigned* bar_count = c.prog;                // count_sync's counter, zeroed before the launch
+    unsigned* seg_count = c.prog + kSegBase;     // the reports' likewise
+    const int first = T.first;
+    const int nseg = nch > (long long)first * nb ? 2 : 1;
+    unsigned bars = 0;                           // device-wide barriers passed in this launch
+    unsigned phases = 0;                         // colour phases before this one
+    // blocks with chunks of report s, and this block's warps there (a round is
+    // one consumer group's: 4 warps)
+    auto seg_blocks = [&](int s) {
+        const long long rest = nch - (s ? (long long)first * nb : 0);
+        return rest < (long long)nb ? (unsigned)rest : nb;
+    };
+    auto seg_warps = [&](int s) {
+        const long long n = s ? mine - first : mine < first ? mine : (long long)first;
+        return n >= 2 ? (unsigned)(kTmaConsumers / 32) : (unsigned)(kTmaGroup / 32);
+    };
     const bool leader = (b == 0 && tid == 0);
     const float sor = c.sor;
     const uint64_t keep = l2_evict_last();
@@ -325,26 +379,18 @@ __global__ void __launch_bounds__(DcLayout<PIPES>::kThreads, DcLayout<PIPES>::kM
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], kTmaGroup / 32);   // one arrival per warp of a group
         }
+        for (int s = 0; s < nseg; ++s) {
+            mbar_init(&seg_bar[s], seg_warps(s));
+            mbar_init(&gate[s], 1);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_err = 0;
     }
     __syncthreads();
     unsigned uses = 0;      // this pipeline's chunks consumed, over all colour phases
     unsigned issued = 0;    // producer: this pipeline's chunks issued, over all phases
-    // producer: chunks of the coming phase whose own parts are already in flight
-    long long primed = 0;
-    const long long pro = pmine < (long long)ring ? pmine : (long long)ring;
-#if TSE_TMA_PREFETCH
-    if (producer && lane == 0) {
-        for (long long j = 0; j < pro; ++j) {
-            const long long m0 = (b + (pipe + j * kPipes) * nb) * C;
-            const long long cnt = (N - m0) < C ? (N - m0) : C;
-            tma_issue_own(c, T, smem + (size_t)(ring0 + j) * T.bytes, &full[ring0 + j], c.K[0], c.D[0],
-                          c.mask[0], m0, cnt);
-        }
-        primed = pro;
-    }
-#endif
+    // the corrections were written by the kernel before (generic stores)
+    if (producer) fence_proxy_async();
 
     for (int inner = 0; inner < c.cycle; ++inner) {
         num_it += 1;
@@ -352,66 +398,72 @@ __global__ void __launch_bounds__(DcLayout<PIPES>::kThreads, DcLayout<PIPES>::kM
         const bool check = c.pressure_schedule ? (num_it < 50 || num_it % 10 == 0) : true;
         if (check) checkno += 1;
         float d2 = 0.0f, dd = 0.0f;
-        bool ok = true;
-        for (int col = 0; col < 2 && ok; ++col) {
+        for (int col = 0; col < 2; ++col, ++phases) {
             const float* Kc = c.K[col];
             float* dw = c.D[col];
             const float* dq = c.D[1 - col];
             const uint8_t* msk = c.mask[col];
             if (producer) {
                 if (lane == 0) {
-                    // the other colour was written (generic stores) before
-                    // the grid barrier; the copies read it through the async proxy
-                    fence_proxy_async();
-                    bool pok = true;
                     for (long long j = 0; j < pmine; ++j, ++issued) {
+                        const int i = pipe + (int)j * kPipes;
+                        bool pok = true;
+                        if (j == 0) pok = mbar_wait_flag(&gate[0], phases & 1u, err);
+                        // the first of this pipeline's rounds past the head
+                        if (nseg > 1 && i >= T.head && i - kPipes < T.head)
+                            pok = pok && mbar_wait_flag(&gate[1], phases & 1u, err);
                         const unsigned s = ring0 + issued % ring;
-                        const long long m0 = (b + (pipe + j * kPipes) * nb) * C;
+                        if (!pok || (issued >= (unsigned)ring &&
+                                     !mbar_wait_flag(&empty[s], (issued / ring - 1) & 1u, err)))
+                            break;
+                        const long long m0 = (b + (long long)i * nb) * C;
+                        const long long cnt = (N - m0) < C ? (N - m0) : C;   // % 32 == 0
                         unsigned char* stg = smem + (size_t)s * T.bytes;
-                        if (j >= primed) {
-                            if (issued >= (unsigned)ring &&
-                                !mbar_wait_flag(&empty[s], (issued / ring - 1) & 1u, err)) {
-                                pok = false;
-                                break;
-                            }
-                            const long long cnt = (N - m0) < C ? (N - m0) : C;   // % 32 == 0
-                            tma_issue_own(c, T, stg, &full[s], Kc, dw, msk, m0, cnt);
-                        }
+                        tma_issue_own(c, T, stg, &full[s], Kc, dw, msk, m0, cnt);
                         tma_issue_windows(c, T, stg, &full[s], dq, m0);
                     }
-                    primed = 0;
-#if TSE_TMA_PREFETCH
-                    // the next phase's own parts (records, r', flags, own
-                    // correction: nothing another block writes) go out as the
-                    // consumers free the stages, before the grid barrier
-                    const int nc = 1 - col;
-                    for (long long j = 0; pok && j < pro; ++j) {
-                        const unsigned v = issued + (unsigned)j;
-                        const unsigned s = ring0 + v % ring;
-                        if (v >= (unsigned)ring &&
-                            !mbar_wait_flag(&empty[s], (v / ring - 1) & 1u, err))
-                            break;
-                        const long long m0 = (b + (pipe + j * kPipes) * nb) * C;
-                        const long long cnt = (N - m0) < C ? (N - m0) : C;
-                        tma_issue_own(c, T, smem + (size_t)s * T.bytes, &full[s], c.K[nc], c.D[nc],
-                                      c.mask[nc], m0, cnt);
-                        primed = j + 1;
-                    }
-#endif
                 }
                 __syncwarp();
+            } else if (gatekeeper) {
+                // the head opens when every block has made the first report of
+                // the phase before, the rest when they have made the second
+                if (lane == 0) {
+                    bool gok = true;
+                    for (int s = 0; gok && s < nseg; ++s) {
+                        gok = seg_wait(seg_count + s * kSegWords, phases * seg_blocks(s), c.bar, err);
+                        // the other colour was written by generic stores; the
+                        // producers' copies read it through the async proxy
+                        fence_proxy_async();
+                        if (gok) mbar_arrive(&gate[s]);
+                    }
+                }
+                __syncwarp();
+            } else if (reporter) {
+                if (lane == 0)
+                    for (int s = 0; s < nseg && mine > (s ? first : 0); ++s) {
+                        if (!mbar_wait_flag(&seg_bar[s], phases & 1u, err)) break;
+                        red_release_add(seg_count + s * kSegWords, 1u);
+                    }
+                __syncwarp();
             } else {
+                bool cok = true;
+                int had = -1;   // the report this warp's last chunk belongs to
                 for (long long j = grank; j < pmine; j += kGroupsPerPipe) {
+                    const int i = pipe + (int)j * kPipes;
+                    const int now = i >= first;
+                    if (had >= 0 && now != had) seg_arrive(&seg_bar[had]);
+                    had = now;
                     const unsigned u = uses + (unsigned)j;
                     const unsigned s = ring0 + u % ring;
                     // warp-uniform: lane 0 waits, the warp follows its outcome,
                     // then every lane observes the completed phase (acquire)
                     int okw = 1;
                     if (lane == 0) okw = mbar_wait_flag(&full[s], (u / ring) & 1u, err);
-                    if (!__shfl_sync(0xffffffffu, okw, 0)) break;
+                    cok = __shfl_sync(0xffffffffu, okw, 0) != 0;
+                    if (!cok) break;
                     mbar_try_wait(&full[s], (u / ring) & 1u);
                     const unsigned char* stg = smem + (size_t)s * T.bytes;
-                    const long long m0 = (b + (pipe + j * kPipes) * nb) * C;
+                    const long long m0 = (b + (long long)i * nb) * C;
                     const int nval = (int)((Nc - m0) < C ? (Nc - m0) : C);
                     // window offsets of cell l of the chunk (32-bit from here on)
                     const int oz = (int)(m0 - ((m0 - H - 1) & ~3LL));
@@ -452,26 +504,22 @@ __global__ void __launch_bounds__(DcLayout<PIPES>::kThreads, DcLayout<PIPES>::kM
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&empty[s]);
                 }
+                if (cok && had >= 0) seg_arrive(&seg_bar[had]);
             }
             uses += (unsigned)pmine;
-            // this phase's stores are read by the next phase's copies
-            fence_proxy_async();
-            __syncthreads();
-            if (*err) { ok = false; break; }   // block-uniform after the barrier
-            if (col == 1 && check) {
-                const double b1 = block_sum<kThreads>((double)d2, sh);
-                const double b3 = block_sum<kThreads>((double)dd, sh);
-                if (tid == 0) {
-                    c.partials[4 * b + 2 * (checkno & 1)] = b1;
-                    c.partials[4 * b + 2 * (checkno & 1) + 1] = b3;
-                }
-            }
-            ok = count_sync(bar_count, ++bars * nb, c.bar);
         }
-        if (!ok) { event = EV_ERROR; break; }
         diff = 1e100;
         bool refresh = false;
         if (check) {
+            __syncthreads();
+            if (*err) { event = EV_ERROR; break; }   // block-uniform after the barrier
+            const double b1 = block_sum<kThreads>((double)d2, sh);
+            const double b3 = block_sum<kThreads>((double)dd, sh);
+            if (tid == 0) {
+                c.partials[4 * b + 2 * (checkno & 1)] = b1;
+                c.partials[4 * b + 2 * (checkno & 1) + 1] = b3;
+            }
+            if (!count_sync(bar_count, ++bars * nb, c.bar)) { event = EV_ERROR; break; }
             double s1 = 0.0, s3 = 0.0;
             for (unsigned q = tid; q < nb; q += blockDim.x) {
                 s1 = s1 + __ldcg(c.partials + 4 * q + 2 * (checkno & 1));
@@ -512,21 +560,15 @@ __global__ void __launch_bounds__(DcLayout<PIPES>::kThreads, DcLayout<PIPES>::kM
         if (halved) { event = EV_HALVE; break; }
         if (refresh) { event = EV_REFRESH; break; }
     }
-    if (producer && lane == 0) {
+    __syncthreads();
+    if (*err) event = EV_ERROR;
+    if (event == EV_ERROR && producer && lane == 0) {
         // every copy this block issued lands before its shared memory is
-        // released (bounded waits, flag ignored): after an error the last
-        // issued use of each stage; primed stages get their missing arrival
-        if (event == EV_ERROR) {
-            atomicExch(&c.bar->error, 1);
-            const unsigned first = issued > (unsigned)ring ? issued - ring : 0u;
-            for (unsigned v = first; v < issued; ++v)
-                mbar_wait_bounded(&full[ring0 + v % ring], (v / ring) & 1u);
-        }
-        for (long long j = 0; j < primed; ++j) {
-            const unsigned v = issued + (unsigned)j;
-            mbar_arrive(&full[ring0 + v % ring]);
-            mbar_wait_bounded(&full[ring0 + v % ring], (v / ring) & 1u);
-        }
+        // released (bounded waits, flag ignored): the last issued use of each
+        // stage
+        atomicExch(&c.bar->error, 1);
+        const unsigned first = issued > (unsigned)ring ? issued - ring : 0u;
+        for (unsigned v = first; v < issued; ++v) mbar_wait_bounded(&full[ring0 + v % ring], (v / ring) & 1u);
     }
     if (leader) {
         st->t = t;
@@ -564,7 +606,7 @@ __global__ void dc_status_kernel(const DcState* st, TseSolveStatus* s) {
 size_t dc_extra_bytes(const Layout& L) {
     long long Ncal = (L.Nc + 31) & ~31LL;
     return 2 * ((size_t)7 * Ncal + (size_t)dc_delta_len(L, Ncal)) * sizeof(float) +
-           align256(sizeof(DcState)) + 256 + 512;
+           align256(sizeof(DcState)) + 256 + align256(kProgBytes);
 }
 
 size_t dc_resident_bytes(const Layout& L) {
@@ -698,7 +740,7 @@ static int run_dc(SolveSetup<Form>& S, double dt, double inc_it, double max_dt, 
         T.stages = st >= 2 * pipes ? st : 0;
     }
     const size_t tma_smem = (size_t)T.stages * T.bytes;
-    const int tma_threads = kTmaConsumers + 32 * pipes;
+    const int tma_threads = pipes == 1 ? DcLayout<1>::kThreads : DcLayout<2>::kThreads;
     const void* tma_k = T.stages > 0 ? tma_kernel(T.stages / pipes, pipes, chunk) : nullptr;
     const int nb_tma = tma_k ? tma_blocks(S.L.Nc, cap, tma_smem, tma_k, tma_threads, chunk) : 0;
     if (opts) {
@@ -708,6 +750,7 @@ static int run_dc(SolveSetup<Form>& S, double dt, double inc_it, double max_dt, 
         opts->ring = nb_tma > 0 ? T.stages / pipes : 0;
     }
     const int nb = nb_tma > 0 ? nb_tma : sweep_blocks(S.L.Nc, cap);
+    if (nb_tma > 0) sweep_head(S.L, nb_tma, T);
     // first_parts > 0: the setup has written the records, r' and that many
     // x^2 partials (the first cycle's scale and residual)
     if (first_parts == 0) {
@@ -737,8 +780,8 @@ static int run_dc(SolveSetup<Form>& S, double dt, double inc_it, double max_dt, 
         }
         void* args[] = {(void*)&c};
         void* targs[] = {(void*)&c, (void*)&T};
-        // staged sweep: its barrier counter starts at 0
-        if (nb_tma > 0 && cudaMemsetAsync(c.prog, 0, sizeof(unsigned), stream) != cudaSuccess) {
+        // staged sweep: its counters start at 0
+        if (nb_tma > 0 && cudaMemsetAsync(c.prog, 0, kProgBytes, stream) != cudaSuccess) {
             rc = TSE_ERR_LAUNCH;
             break;
         }

@@ -43,7 +43,7 @@ struct DcCtl {
     double* partials;    // sweep kernel: 4 per block; residual kernel: 1 per block
     GridBarrier* bar;
     DcState* st;
-    unsigned* prog;      // staged sweep: its barrier counter
+    unsigned* prog;      // staged sweep: its barrier counter, then its reports' (kProgBytes)
 };
 
 // K'_q = k_q / Den of one cell (6 FP32 values, one 24-byte record)
@@ -259,7 +259,40 @@ struct TmaStage {
     int lz, lx;   // window lengths in floats
     int stages;   // stages of the launch, over all its pipelines (set by the launcher)
     int chunk;    // cells a chunk (256, 512 or 1024)
+    int head;     // single-model sweep: rounds a phase begins with early, and
+    int first;    // rounds its first report covers (sweep_head)
 };
+
+// Phases of the single-model sweep overlap.  Block b takes chunks b, b + nb,
+// ...; its i-th chunk is round i.  A chunk's windows reach `reach` cells, so at
+// most `far` rounds, to either side; the `head` first rounds of a phase may
+// therefore begin once all blocks have done the `first` = head + far first
+// rounds of the phase before, and only the rest needs all of it.  Two reports
+// a phase: rounds [0, first) and the others.
+//
+// head: long enough that a phase's last chunks are done and reported (a few
+// microseconds) while the next one's head is swept, short enough that the
+// first report is old by then (8 rounds: 25.0 us an iteration at 192 x 192 x
+// 128 and 85-86 at 320 x 320 x 160; 16: 23.3 and 83; 32: 23.3 and 82-86).
+#ifndef TSE_HEAD
+#define TSE_HEAD 16
+#endif
+constexpr int kHead = TSE_HEAD;
+inline void sweep_head(const Layout& L, long long nb, TmaStage& T) {
+    const long long nch = (L.Nc + T.chunk - 1) / T.chunk, rounds = (nch + nb - 1) / nb;
+    const long long reach = L.SX + L.H + T.chunk + 16, cells = nb * T.chunk;
+    long long far = (reach + cells - 1) / cells;
+    far += far & 1;   // even: whole pairs of rounds, one a pipeline
+    long long h = (rounds - far) / 2;
+    h = h > kHead ? kHead : h < 2 ? 2 : h;
+    T.head = (int)(h & ~1LL);
+    T.first = T.head + (int)far;
+}
+constexpr int kSegs = 2;
+// words from the barrier counter to report s's counter (a sector each)
+constexpr int kSegWords = 8, kSegBase = 32;
+constexpr size_t kProgBytes = (kSegBase + kSegs * kSegWords) * sizeof(unsigned);
+
 
 __host__ __device__ inline TmaStage tma_stage(int H, int C = kTmaChunk) {
     TmaStage t;
@@ -280,14 +313,10 @@ __host__ __device__ inline TmaStage tma_stage(int H, int C = kTmaChunk) {
     return t;
 }
 
-// Chunk q of the colour being swept, in two parts.  The first part (records,
-// r', flags, the chunk's own old correction) depends on nothing another block
-// writes during the launch -- the old correction of a chunk is written only
-// by the block that owns the chunk -- so it may be issued before the grid
-// barrier that ends the previous phase; it adds its bytes to the stage's
-// transaction count without arriving.  The second part (the three windows of
-// the other colour, which other blocks have just written) is issued after the
-// barrier and carries the stage's single arrival.
+// Chunk q of the colour being swept, in two parts: records, r', flags and the
+// chunk's own old correction, which add their bytes to the stage's transaction
+// count without arriving, and the three windows of the other colour, which
+// carry the stage's single arrival.
 __device__ __forceinline__ void tma_issue_own_n(long long N, const TmaStage& T, unsigned char* stage,
                                                 uint64_t* bar, const float* Kc, const float* dw,
                                                 const uint8_t* msk, long long m0, long long cnt) {
