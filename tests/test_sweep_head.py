@@ -114,3 +114,24 @@ def test_phases_follow_each_other_without_a_barrier():
                     arrived[b][s] += 1
                 idle = 0
         assert all(count[s] <= phases * blocks[s] for s in range(nseg))
+
+
+def test_record_blocks_are_aligned_and_inside_their_array():
+    """A chunk's record block (records, r', flags) is one copy: 16-byte
+    aligned, a multiple of 16 bytes, inside the colour's array for every
+    compiled chunk size, and every cell's parts lie where the copy puts them."""
+    rng = random.Random(3)
+    for Nc in [1, 2, 255, 256, 257, 511, 512, 1023, 1024, 1025] + [rng.randint(1, 200000) for _ in range(40)]:
+        floats = ((Nc + 1023) >> 10) * (29 << 8)
+        assert 2 * floats * 4 % 16 == 0            # the second colour and the corrections after it
+        for ks in (8, 9, 10):
+            C, block = 1 << ks, 29 << (ks - 2)
+            assert block * 4 % 16 == 0 and block * 4 == 29 * C
+            for q in range(-(-Nc // C)):
+                assert (q + 1) * block <= floats
+            for m in (0, Nc // 2, Nc - 1):
+                o = m & (C - 1)
+                base = (m >> ks) * block
+                rec, rp, flag = base + 6 * o, base + 6 * C + o, 4 * (base + 7 * C) + o
+                assert rec * 4 % 8 == 0 and rec + 6 <= base + 6 * C
+                assert rp < base + 7 * C and flag < 4 * (base + block)

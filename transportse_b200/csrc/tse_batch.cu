@@ -138,7 +138,7 @@ __device__ void cluster_dc_solve(cg::cluster_group& cl, const BatchItem<Form>& i
                     const double r = F.sum(col, m, f, Xo) - den * x;
                     rp = (float)(r / den);
                 }
-                Kc[6 * N + m] = rp;
+                *k_rp(Kc, c.ks, m) = rp;
                 Dc[m] = 0.0f;
             }
         }
@@ -168,7 +168,7 @@ __device__ void cluster_dc_solve(cg::cluster_group& cl, const BatchItem<Form>& i
                     const bool va = ma < Nc;
                     const long long la = va ? ma : Nc - 1;
                     Cell a;
-                    load_cell(a, Kc, dw, dq, msk, la, N, SX, H);
+                    load_cell(a, Kc, dw, dq, msk, la, c.ks, SX, H);
                     const float na = relax(a, dq, la, Nc, sor);
                     if (va) {
                         dw[ma] = na;
@@ -541,8 +541,8 @@ __device__ __forceinline__ void fused_sweep_body(const FusedArgs& A, const TmaSt
                                 h.H = c.L.H;
                                 h.sor = c.sor;
                                 hdr[s] = h;
-                                tma_issue_own_n(c.Ncal, T, stg, &full[s], c.K[col], c.D[col], c.mask[col], m0,
-                                                cnt);
+                                tma_issue_own(T, stg, &full[s], k_block((const float*)c.K[col], kTmaChunkLog2, m0),
+                                              c.D[col] + m0, cnt);
                                 tma_issue_windows_n(h.SX, h.H, T, stg, &full[s], c.D[1 - col], m0);
                                 ++issued;
                             }

@@ -55,12 +55,20 @@ constexpr int kSweepBlock = TSE_SWEEP_BLOCK;
 // 96^3 to 256 x 256 x 128.)
 constexpr int kDcPipes = 2;
 constexpr int kDcMaxRing = 4;
-template <int PIPES>
+//
+// Consumers: 8 warps, or 16 (WIDE, two pipelines) where the solve's state stays
+// in L2 and the chunks arrive faster than 8 warps relax them.  Measured, us per
+// iteration with 8 and with 16: 128^3 14.8 and 13.5, 192 x 192 x 128 22.5 and
+// 22.2, whole 256 x 256 x 128 solves at the power cap 460 and 467 ms.
+template <int PIPES, bool WIDE = false>
 struct DcLayout {
-    static constexpr int kThreads = kTmaConsumers + 32 * PIPES + 64;   // consumers, producers, reporter, gatekeeper
+    static_assert(!WIDE || PIPES == 2, "one pipeline runs two blocks per SM");
+    static constexpr int kConsumers = WIDE ? 2 * kTmaConsumers : kTmaConsumers;
+    static constexpr int kThreads = kConsumers + 32 * PIPES + 64;   // consumers, producers, reporter, gatekeeper
     static constexpr int kMinBlocks = PIPES == 1 ? 2 : 1;
-    static constexpr int kGroupsPerPipe = (kTmaConsumers / kTmaGroup) / PIPES;
-    static_assert((kTmaConsumers / kTmaGroup) % PIPES == 0, "every pipeline has its own consumer groups");
+    static constexpr int kGroups = kConsumers / kTmaGroup;
+    static constexpr int kGroupsPerPipe = kGroups / PIPES;
+    static_assert(kGroups % PIPES == 0, "every pipeline has its own consumer groups");
 };
 
 // ------------------------------------------------------------ FP64 kernels
@@ -171,7 +179,7 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) dc_sweep_kernel(
     __shared__ double sh[kSweepBlock / 32];
     __shared__ double s_val;
     const unsigned nb = gridDim.x;
-    const long long Nc = c.L.Nc, N = c.Ncal, SX = c.L.SX;
+    const long long Nc = c.L.Nc, SX = c.L.SX;
     const int H = c.L.H;
     const int lane = threadIdx.x & 31;
     const long long end = Nc;
@@ -208,7 +216,7 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) dc_sweep_kernel(
                 const bool va = ma < end;
                 const long long la = va ? ma : end - 1;
                 Cell a;
-                load_cell(a, Kc, dw, dq, msk, la, N, SX, H);
+                load_cell(a, Kc, dw, dq, msk, la, c.ks, SX, H);
                 const float na = relax(a, dq, la, end, sor);
                 if (va) {
                     dw[ma] = na;
@@ -284,11 +292,12 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) dc_sweep_kernel(
 // these steps on a consumer's or a producer's path made the sweep slower than
 // the device-wide barrier did (consumers' fences 2.5 times, the producers'
 // polls 1.5 times, the producers' proxy fences 1.2 times).  Bound: DRAM, 29
-// bytes an update, and below about 3M cells the producers' issue rate (7 copies
-// a chunk, 100 ns each).  Barrier after every phase and now, us per iteration
+// bytes an update, and at the power cap's clocks the producers' issue rate (5
+// copies a chunk) and the consumers'.  Barrier after every phase and now, us per iteration
 // of the sweep alone (B200, both on one box, twice): 128^3 15.2 -> 14.6, 192 x
 // 192 x 128 26.2 -> 23.3, 256 x 256 x 128 42.0-42.8 -> 39.7-42.3 (0.94 of the
-// measured HBM rate at best), 320 x 320 x 160 88.3 -> 82.6-83.5.
+// measured HBM rate at best), 320 x 320 x 160 88.3 -> 82.6-83.5; with the record
+// blocks and 8 or 16 consumer warps 13.5, 22.2, 38.8-41.2 and 83.4-86.
 // seg_wait: a report's count has reached `target` (acquire); bounded.
 __device__ __forceinline__ bool seg_wait(const unsigned* count, unsigned target, GridBarrier* bar,
                                          volatile int* err) {
@@ -313,13 +322,14 @@ __device__ __forceinline__ void seg_arrive(uint64_t* bar) {
     if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
 }
 
-template <int RING, int PIPES, int CHUNK>
-__global__ void __launch_bounds__(DcLayout<PIPES>::kThreads, DcLayout<PIPES>::kMinBlocks)
+template <int RING, int PIPES, int CHUNK, bool WIDE>
+__global__ void __launch_bounds__(DcLayout<PIPES, WIDE>::kThreads, DcLayout<PIPES, WIDE>::kMinBlocks)
     dc_sweep_tma_kernel(DcCtl c, TmaStage T) {
     static_assert(CHUNK % kTmaGroup == 0 && CHUNK <= kDcMaxChunk, "whole cells per thread, in the margins");
     constexpr int kCellsPerThread = CHUNK / kTmaGroup;
     constexpr int kPipes = PIPES;
-    constexpr int kThreads = DcLayout<PIPES>::kThreads;
+    constexpr int kThreads = DcLayout<PIPES, WIDE>::kThreads;
+    constexpr int kConsumers = DcLayout<PIPES, WIDE>::kConsumers;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t full[RING * PIPES];
     __shared__ __align__(8) uint64_t empty[RING * PIPES];
@@ -329,16 +339,16 @@ __global__ void __launch_bounds__(DcLayout<PIPES>::kThreads, DcLayout<PIPES>::kM
     const unsigned nb = gridDim.x, b = blockIdx.x;
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
-    const bool reporter = warp == kTmaConsumers / 32 + kPipes;
-    const bool gatekeeper = warp == kTmaConsumers / 32 + kPipes + 1;
-    const bool producer = !reporter && !gatekeeper && warp >= kTmaConsumers / 32;
-    const int group = tid / kTmaGroup;                  // consumers: 0 or 1
+    const bool reporter = warp == kConsumers / 32 + kPipes;
+    const bool gatekeeper = warp == kConsumers / 32 + kPipes + 1;
+    const bool producer = !reporter && !gatekeeper && warp >= kConsumers / 32;
+    const int group = tid / kTmaGroup;                  // consumers: 0, 1, ...
     const int gt = tid & (kTmaGroup - 1);               // thread within its group
     // this thread's pipeline (producer warp + its ring of stages +
     // its consumer groups), and a consumer group's rank within it
-    const int pipe = producer ? warp - kTmaConsumers / 32 : group % kPipes;
+    const int pipe = producer ? warp - kConsumers / 32 : group % kPipes;
     const int grank = group / kPipes;
-    constexpr int kGroupsPerPipe = DcLayout<PIPES>::kGroupsPerPipe;
+    constexpr int kGroupsPerPipe = DcLayout<PIPES, WIDE>::kGroupsPerPipe;
     constexpr unsigned ring = RING;                     // stages of a ring (T.stages / PIPES)
     const unsigned ring0 = (unsigned)pipe * ring;    // the pipeline's first stage
     const long long Nc = c.L.Nc, N = c.Ncal, SX = c.L.SX, C = CHUNK;
@@ -361,7 +371,8 @@ __global__ void __launch_bounds__(DcLayout<PIPES>::kThreads, DcLayout<PIPES>::kM
     };
     auto seg_warps = [&](int s) {
         const long long n = s ? mine - first : mine < first ? mine : (long long)first;
-        return n >= 2 ? (unsigned)(kTmaConsumers / 32) : (unsigned)(kTmaGroup / 32);
+        const int groups = DcLayout<PIPES, WIDE>::kGroups;
+        return (unsigned)((n < groups ? (int)n : groups) * (kTmaGroup / 32));
     };
     const bool leader = (b == 0 && tid == 0);
     const float sor = c.sor;
@@ -402,7 +413,6 @@ __global__ void __launch_bounds__(DcLayout<PIPES>::kThreads, DcLayout<PIPES>::kM
             const float* Kc = c.K[col];
             float* dw = c.D[col];
             const float* dq = c.D[1 - col];
-            const uint8_t* msk = c.mask[col];
             if (producer) {
                 if (lane == 0) {
                     for (long long j = 0; j < pmine; ++j, ++issued) {
@@ -416,10 +426,9 @@ __global__ void __launch_bounds__(DcLayout<PIPES>::kThreads, DcLayout<PIPES>::kM
                         if (!pok || (issued >= (unsigned)ring &&
                                      !mbar_wait_flag(&empty[s], (issued / ring - 1) & 1u, err)))
                             break;
-                        const long long m0 = (b + (long long)i * nb) * C;
-                        const long long cnt = (N - m0) < C ? (N - m0) : C;   // % 32 == 0
+                        const long long q = b + (long long)i * nb, m0 = q * C;
                         unsigned char* stg = smem + (size_t)s * T.bytes;
-                        tma_issue_own(c, T, stg, &full[s], Kc, dw, msk, m0, cnt);
+                        tma_issue_own(T, stg, &full[s], Kc + q * (29 * CHUNK / 4), dw + m0, (N - m0) < C ? (N - m0) : C);
                         tma_issue_windows(c, T, stg, &full[s], dq, m0);
                     }
                 }
@@ -455,6 +464,9 @@ __global__ void __launch_bounds__(DcLayout<PIPES>::kThreads, DcLayout<PIPES>::kM
                     had = now;
                     const unsigned u = uses + (unsigned)j;
                     const unsigned s = ring0 + u % ring;
+                    const long long m0 = (b + (long long)i * nb) * C;
+                    const int nval = (int)((Nc - m0) < C ? (Nc - m0) : C);
+                    float* out = dw + m0;
                     // warp-uniform: lane 0 waits, the warp follows its outcome,
                     // then every lane observes the completed phase (acquire)
                     int okw = 1;
@@ -463,8 +475,6 @@ __global__ void __launch_bounds__(DcLayout<PIPES>::kThreads, DcLayout<PIPES>::kM
                     if (!cok) break;
                     mbar_try_wait(&full[s], (u / ring) & 1u);
                     const unsigned char* stg = smem + (size_t)s * T.bytes;
-                    const long long m0 = (b + (long long)i * nb) * C;
-                    const int nval = (int)((Nc - m0) < C ? (Nc - m0) : C);
                     // window offsets of cell l of the chunk (32-bit from here on)
                     const int oz = (int)(m0 - ((m0 - H - 1) & ~3LL));
                     const int oxp = (int)(m0 + SX - ((m0 + SX) & ~3LL));
@@ -476,7 +486,6 @@ __global__ void __launch_bounds__(DcLayout<PIPES>::kThreads, DcLayout<PIPES>::kM
                     const float* wz = reinterpret_cast<const float*>(stg + T.wz);
                     const float* wxp = reinterpret_cast<const float*>(stg + T.wxp);
                     const float* wxm = reinterpret_cast<const float*>(stg + T.wxm);
-                    float* out = dw + m0;
 #pragma unroll
                     for (int r = 0; r < kCellsPerThread; ++r) {
                         const int l = gt + r * kTmaGroup;
@@ -604,8 +613,8 @@ __global__ void dc_status_kernel(const DcState* st, TseSolveStatus* s) {
 
 // ------------------------------------------------------------------ host
 size_t dc_extra_bytes(const Layout& L) {
-    long long Ncal = (L.Nc + 31) & ~31LL;
-    return 2 * ((size_t)7 * Ncal + (size_t)dc_delta_len(L, Ncal)) * sizeof(float) +
+    const long long Ncal = (L.Nc + 31) & ~31LL;
+    return 2 * ((size_t)k_floats(L) + (size_t)dc_delta_len(L, Ncal)) * sizeof(float) +
            align256(sizeof(DcState)) + 256 + align256(kProgBytes);
 }
 
@@ -652,18 +661,33 @@ static size_t tma_max_smem() {
 // grid's windows do not fit (the plain sweep kernel runs instead)
 // the instantiation for rings of `ring` stages (2 .. 4), `pipes` pipelines
 // per block (1: two blocks per SM) and chunks of `chunk` cells
-template <int PIPES, int CHUNK>
+template <int PIPES, int CHUNK, bool WIDE>
 static const void* tma_kernel_r(int ring) {
-    return ring <= 2 ? (const void*)dc_sweep_tma_kernel<2, PIPES, CHUNK>
-         : ring == 3 ? (const void*)dc_sweep_tma_kernel<3, PIPES, CHUNK>
-                     : (const void*)dc_sweep_tma_kernel<4, PIPES, CHUNK>;
+    return ring <= 2 ? (const void*)dc_sweep_tma_kernel<2, PIPES, CHUNK, WIDE>
+         : ring == 3 ? (const void*)dc_sweep_tma_kernel<3, PIPES, CHUNK, WIDE>
+                     : (const void*)dc_sweep_tma_kernel<4, PIPES, CHUNK, WIDE>;
 }
-static const void* tma_kernel(int ring, int pipes, int chunk) {
-    if (pipes == 1)
-        return chunk == 256 ? tma_kernel_r<1, 256>(ring) : chunk == 1024 ? tma_kernel_r<1, 1024>(ring)
-                                                                         : tma_kernel_r<1, 512>(ring);
-    return chunk == 256 ? tma_kernel_r<2, 256>(ring) : chunk == 1024 ? tma_kernel_r<2, 1024>(ring)
-                                                                     : tma_kernel_r<2, 512>(ring);
+template <int PIPES, bool WIDE>
+static const void* tma_kernel_c(int ring, int chunk) {
+    return chunk == 256 ? tma_kernel_r<PIPES, 256, WIDE>(ring)
+         : chunk == 1024 ? tma_kernel_r<PIPES, 1024, WIDE>(ring)
+                         : tma_kernel_r<PIPES, 512, WIDE>(ring);
+}
+static const void* tma_kernel(int ring, int pipes, int chunk, bool wide) {
+    return pipes == 1 ? tma_kernel_c<1, false>(ring, chunk)
+         : wide ? tma_kernel_c<2, true>(ring, chunk)
+                : tma_kernel_c<2, false>(ring, chunk);
+}
+// 16 consumer warps where a solve's records and corrections (33 bytes a cell)
+// fit in L2
+static bool tma_wide(long long Nc, int pipes) {
+    int dev = 0, l2 = 0;
+    if (pipes != 2 || cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return 2 * Nc * 33 <= (long long)l2;
 }
 
 static int tma_blocks(long long Nc, int cap, size_t smem, const void* kernel, int threads, int chunk) {
@@ -688,6 +712,11 @@ static int tma_blocks(long long Nc, int cap, size_t smem, const void* kernel, in
     if (nb > kMaxBlocks / 2) nb = kMaxBlocks / 2;
     if (cap > 0 && nb > cap) nb = cap;
     return nb < 1 ? 1 : (int)nb;
+}
+
+// the record blocks' cells: the chunk the call's options name (512 otherwise)
+static int dc_block_log2(const TseDcOptions* opts) {
+    return opts && opts->chunk == 256 ? 8 : opts && opts->chunk == 1024 ? 10 : 9;
 }
 
 template <class Form>
@@ -728,7 +757,7 @@ static int run_dc(SolveSetup<Form>& S, double dt, double inc_it, double max_dt, 
     // the staged sweep's variant: chunk size, pipelines per block and ring
     // length from the call's options (0: 512 cells, 2 pipelines, as many
     // stages as fit up to 4 a ring)
-    const int chunk = (opts && (opts->chunk == 256 || opts->chunk == 1024)) ? opts->chunk : 512;
+    const int chunk = 1 << S.ks;
     const int pipes = (opts && opts->pipes == 1) ? 1 : kDcPipes;
     const int want_ring = (opts && opts->ring >= 2 && opts->ring <= kDcMaxRing) ? opts->ring : kDcMaxRing;
     TmaStage T = tma_stage(S.L.H, chunk);
@@ -740,8 +769,11 @@ static int run_dc(SolveSetup<Form>& S, double dt, double inc_it, double max_dt, 
         T.stages = st >= 2 * pipes ? st : 0;
     }
     const size_t tma_smem = (size_t)T.stages * T.bytes;
-    const int tma_threads = pipes == 1 ? DcLayout<1>::kThreads : DcLayout<2>::kThreads;
-    const void* tma_k = T.stages > 0 ? tma_kernel(T.stages / pipes, pipes, chunk) : nullptr;
+    const bool wide = tma_wide(S.L.Nc, pipes);
+    const int tma_threads = pipes == 1 ? DcLayout<1>::kThreads
+                            : wide     ? DcLayout<2, true>::kThreads
+                                       : DcLayout<2>::kThreads;
+    const void* tma_k = T.stages > 0 ? tma_kernel(T.stages / pipes, pipes, chunk, wide) : nullptr;
     const int nb_tma = tma_k ? tma_blocks(S.L.Nc, cap, tma_smem, tma_k, tma_threads, chunk) : 0;
     if (opts) {
         // the variant that ran (0 when the plain-load sweep did)
@@ -924,6 +956,7 @@ extern "C" int32_t tse_compute_P_dc(const TseGrid* grid, const TsePressureArgs* 
         return TSE_ERR_ARG;
     cudaStream_t stream = (cudaStream_t)stream_;
     PressureSetup S;
+    S.ks = dc_block_log2(opts);
     int nparts = 0;
     int rc = setup_pressure_dc(grid, args, d_ws, ws_bytes, stream, S, &nparts);
     if (rc != TSE_OK) return rc;
@@ -942,6 +975,7 @@ extern "C" int32_t tse_compute_C_dc(const TseGrid* grid, const TseSpeciesArgs* a
         return TSE_ERR_ARG;
     cudaStream_t stream = (cudaStream_t)stream_;
     TransportSetup S;
+    S.ks = dc_block_log2(opts);
     int nparts = 0;
     int rc = setup_species_dc(grid, a, d_ws, ws_bytes, stream, S, &nparts);
     if (rc != TSE_OK) return rc;
@@ -960,6 +994,7 @@ extern "C" int32_t tse_compute_T_dc(const TseGrid* grid, const TseHeatArgs* a,
         return TSE_ERR_ARG;
     cudaStream_t stream = (cudaStream_t)stream_;
     TransportSetup S;
+    S.ks = dc_block_log2(opts);
     int nparts = 0;
     int rc = setup_heat_dc(grid, a, d_ws, ws_bytes, stream, S, &nparts);
     if (rc != TSE_OK) return rc;

@@ -37,7 +37,8 @@ struct DcCtl {
     float sor;
     double* X[2];        // FP64 iterate per colour
     const uint8_t* mask[2];
-    float* K[2];         // per colour: Ncal 24-byte coefficient records, then Ncal r'
+    float* K[2];         // per colour: record blocks (k_rec, k_rp, k_flag)
+    int ks;              // log2 of a block's cells
     float* D[2];         // per colour: correction, valid on [-G, Nc + G); the
                          // margins stay 0 so neighbour loads need no guard
     double* partials;    // sweep kernel: 4 per block; residual kernel: 1 per block
@@ -46,10 +47,39 @@ struct DcCtl {
     unsigned* prog;      // staged sweep: its barrier counter, then its reports' (kProgBytes)
 };
 
+// What a half-sweep streams of a cell -- its 24-byte coefficient record, r' and
+// flag byte -- lies in blocks of 2^ks cells, a block's records first, then its
+// r', then its flags, so that a chunk of that many cells is one contiguous
+// copy.  (As three arrays, three copies a chunk: a producer warp issues copies
+// one after another, about 100 ns each at full clock.)
+__host__ __device__ inline long long k_block_floats(int ks) { return 29LL << (ks - 2); }
+// floats per colour, for any block size up to 1024 cells
+__host__ __device__ inline long long k_floats(const Layout& L) {
+    return ((L.Nc + 1023) >> 10) * k_block_floats(10);
+}
+template <class T>
+__device__ __forceinline__ T* k_block(T* K, int ks, long long m) {
+    return K + (m >> ks) * k_block_floats(ks);
+}
+__device__ __forceinline__ float2* k_rec(float* K, int ks, long long m) {
+    return reinterpret_cast<float2*>(k_block(K, ks, m) + 6 * (m & ((1LL << ks) - 1)));
+}
+__device__ __forceinline__ const float2* k_rec(const float* K, int ks, long long m) {
+    return reinterpret_cast<const float2*>(k_block(K, ks, m) + 6 * (m & ((1LL << ks) - 1)));
+}
+template <class T>
+__device__ __forceinline__ T* k_rp(T* K, int ks, long long m) {
+    return k_block(K, ks, m) + (6LL << ks) + (m & ((1LL << ks) - 1));
+}
+__device__ __forceinline__ uint8_t* k_flag(float* K, int ks, long long m) {
+    return reinterpret_cast<uint8_t*>(k_block(K, ks, m) + (7LL << ks)) + (m & ((1LL << ks) - 1));
+}
+
 // K'_q = k_q / Den of one cell (6 FP32 values, one 24-byte record)
 template <class Form>
 __device__ __forceinline__ void scale_cell(const Form& F, const DcCtl& c, int col, long long m) {
-    float2* rec = reinterpret_cast<float2*>(c.K[col] + 6 * m);
+    float2* rec = k_rec(c.K[col], c.ks, m);
+    *k_flag(c.K[col], c.ks, m) = c.mask[col][m];
     if (c.mask[col][m] & F_ACTIVE) {
         const double den = F.den(col, m);
 #pragma unroll
@@ -90,7 +120,7 @@ __device__ __forceinline__ double residual_block_cells(const Form& F, const DcCt
             const double r = F.sum(col, m, f, c.X[1 - col]) - den * x;
             rp = (float)(r / den);
         }
-        c.K[col][6 * c.Ncal + m] = rp;
+        *k_rp(c.K[col], c.ks, m) = rp;
         c.D[col][m] = 0.0f;
     }
     return o2;
@@ -109,12 +139,12 @@ struct Cell {
 
 __device__ __forceinline__ void load_cell(Cell& a, const float* __restrict__ Kc, const float* dw,
                                           const float* dq, const uint8_t* __restrict__ msk,
-                                          long long m, long long N, long long SX, int H) {
-    const float2* rec = reinterpret_cast<const float2*>(Kc + 6 * m);
+                                          long long m, int ks, long long SX, int H) {
+    const float2* rec = k_rec(Kc, ks, m);
     a.k01 = rec[0];
     a.k23 = rec[1];
     a.k45 = rec[2];
-    a.r = Kc[6 * N + m];
+    a.r = *k_rp(Kc, ks, m);
     a.odd = (msk[m] & F_KODD) != 0;
     a.old = dw[m];
     a.xp = __ldcg(dq + m + SX);
@@ -141,7 +171,7 @@ __device__ __forceinline__ float relax(const Cell& a, const float* dq, long long
     return fmaf(sor, acc - a.old, a.old);
 }
 
-// FP32 arrays: per colour 7 * Ncal floats (records + r'), then the
+// FP32 arrays: per colour the record blocks (k_floats), then the
 // correction with margins of G >= SX + 1, then the state record and the
 // staged sweep's barrier counter.  The margins also hold the neighbour windows that the
 // staged sweep copies for a chunk of up to kDcMaxChunk cells at either end
@@ -175,7 +205,7 @@ int dc_begin_fused(const DcCtl& c, double dt, int nparts, cudaStream_t stream);
 // this form: 1/Den is formed once.
 struct DcFuse {
     float* K[2];
-    long long Ncal;
+    int ks;
     double* partials;
     int per_thread;   // cells a thread assembles (blocks of kBlock consecutive cells)
 };
@@ -215,9 +245,10 @@ inline void dc_carve(SolveSetup<Form>& S, DcCtl& c, int x_index) {
     c.mask[1] = S.mask[1];
     float* base = (float*)(((uintptr_t)S.tail + 255) & ~(uintptr_t)255);
     const long long G = dc_margin(S.L), dlen = dc_delta_len(S.L, S.Ncal);
+    c.ks = S.ks;
     c.K[0] = base;
-    c.K[1] = base + (size_t)7 * S.Ncal;
-    float* dbase = base + (size_t)14 * S.Ncal;
+    c.K[1] = base + k_floats(S.L);
+    float* dbase = base + 2 * k_floats(S.L);
     c.D[0] = dbase + G;
     c.D[1] = dbase + dlen + G;
     c.st = (DcState*)(dbase + 2 * dlen);
@@ -249,6 +280,8 @@ inline void dc_carve(SolveSetup<Form>& S, DcCtl& c, int x_index) {
 #define TSE_TMA_MINB 2
 #endif
 constexpr int kTmaChunk = TSE_TMA_CHUNK;
+constexpr int kTmaChunkLog2 = 9;
+static_assert(kTmaChunk == 1 << kTmaChunkLog2, "a chunk is a record block");
 constexpr int kTmaStages = TSE_TMA_STAGES;
 static_assert(kTmaChunk % 32 == 0, "chunk: 16-byte copies of every array");
 static_assert(kTmaChunk <= kDcMaxChunk, "windows must stay inside the correction margins");
@@ -313,27 +346,17 @@ __host__ __device__ inline TmaStage tma_stage(int H, int C = kTmaChunk) {
     return t;
 }
 
-// Chunk q of the colour being swept, in two parts: records, r', flags and the
-// chunk's own old correction, which add their bytes to the stage's transaction
-// count without arriving, and the three windows of the other colour, which
-// carry the stage's single arrival.
-__device__ __forceinline__ void tma_issue_own_n(long long N, const TmaStage& T, unsigned char* stage,
-                                                uint64_t* bar, const float* Kc, const float* dw,
-                                                const uint8_t* msk, long long m0, long long cnt) {
-    const unsigned b_rec = (unsigned)(24 * cnt), b_rp = (unsigned)(4 * cnt), b_msk = (unsigned)cnt,
-                   b_dw = (unsigned)(4 * cnt);
-    const uint64_t first = l2_evict_first(), last = l2_evict_last();
-    mbar_add_tx(bar, b_rec + b_rp + b_msk + b_dw);
-    bulk_g2s_hint(stage + T.rec, Kc + 6 * m0, b_rec, bar, first);
-    bulk_g2s_hint(stage + T.rp, Kc + 6 * N + m0, b_rp, bar, first);
-    bulk_g2s_hint(stage + T.msk, msk + m0, b_msk, bar, first);
-    bulk_g2s_hint(stage + T.dw, dw + m0, b_dw, bar, last);
-}
-
-__device__ __forceinline__ void tma_issue_own(const DcCtl& c, const TmaStage& T, unsigned char* stage,
-                                              uint64_t* bar, const float* Kc, const float* dw,
-                                              const uint8_t* msk, long long m0, long long cnt) {
-    tma_issue_own_n(c.Ncal, T, stage, bar, Kc, dw, msk, m0, cnt);
+// A chunk of the colour being swept, in two parts: its record block and (where
+// the consumers do not read it themselves) its own old correction, which add
+// their bytes to the stage's transaction count without arriving, and the three
+// windows of the other colour, which carry the stage's single arrival.  The
+// block is copied whole; dw: cnt cells from the chunk's first, or null.
+__device__ __forceinline__ void tma_issue_own(const TmaStage& T, unsigned char* stage, uint64_t* bar,
+                                              const float* block, const float* dw, long long cnt) {
+    const unsigned b_blk = (unsigned)(29 * T.chunk), b_dw = dw ? (unsigned)(4 * cnt) : 0u;
+    mbar_add_tx(bar, b_blk + b_dw);
+    bulk_g2s_hint(stage + T.rec, block, b_blk, bar, l2_evict_first());
+    if (dw) bulk_g2s_hint(stage + T.dw, dw, b_dw, bar, l2_evict_last());
 }
 
 __device__ __forceinline__ void tma_issue_windows_n(long long SX, int H, const TmaStage& T,

@@ -160,11 +160,11 @@ __global__ void __launch_bounds__(NT, 1)
                     float2 a01 = make_float2(0.0f, 0.0f), a23 = a01, a45 = a01;
                     float rr = 0.0f;
                     if (used && 4 * gg + q < H) {
-                        const float2* rec = reinterpret_cast<const float2*>(Kc + 6 * (m0 + q));
+                        const float2* rec = k_rec(Kc, c.ks, m0 + q);
                         a01 = __ldcg(rec);
                         a23 = __ldcg(rec + 1);
                         a45 = __ldcg(rec + 2);
-                        rr = __ldcg(Kc + 6 * c.Ncal + m0 + q);
+                        rr = __ldcg(k_rp(Kc, c.ks, m0 + q));
                     }
                     k[col][g][q][0] = a01.x;
                     k[col][g][q][1] = a01.y;
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(NT, 1)
                     const double den = F.den(col, m);
                     rp = (float)((F.sum(col, m, f, col ? c.X[0] : c.X[1]) - den * x) / den);
                 }
-                (col ? c.K[1] : c.K[0])[6 * c.Ncal + m] = rp;
+                *k_rp(col ? c.K[1] : c.K[0], c.ks, m) = rp;
             }
         }
         x2 = o2;

@@ -241,6 +241,7 @@ struct SolveSetup {
     char* tail;          // workspace bytes after the exact form's arrays
     size_t tail_bytes;
     double* faces = nullptr;   // transport: the face pass's values
+    int ks = 9;          // mixed-precision form: log2 of the record blocks' cells
 };
 using PressureSetup = SolveSetup<PressureForm>;
 using TransportSetup = SolveSetup<TransportForm>;

@@ -50,9 +50,10 @@ __device__ __forceinline__ double assemble_p_cell(const TseGrid& g, const TsePre
         for (int q = 0; q < PA_COUNT; ++q) b[q * N + m] = 0.0;
         msk[m] = 0;
         if (DC) {
-            float2* rec = reinterpret_cast<float2*>(fz.K[col] + 6 * m);
+            float2* rec = k_rec(fz.K[col], fz.ks, m);
             for (int q = 0; q < 3; ++q) rec[q] = make_float2(0.0f, 0.0f);
-            fz.K[col][6 * fz.Ncal + m] = 0.0f;
+            *k_rp(fz.K[col], fz.ks, m) = 0.0f;
+            *k_flag(fz.K[col], fz.ks, m) = 0;
         }
         return 0.0;
     }
@@ -119,7 +120,7 @@ __device__ __forceinline__ double assemble_p_cell(const TseGrid& g, const TsePre
     if (active) f |= F_ACTIVE;
     msk[m] = f;
     if (DC) {
-        float2* rec = reinterpret_cast<float2*>(fz.K[col] + 6 * m);
+        float2* rec = k_rec(fz.K[col], fz.ks, m);
         float rp = 0.0f;
         if (active) {
             const double rden = 1.0 / DEN;
@@ -153,7 +154,8 @@ __device__ __forceinline__ double assemble_p_cell(const TseGrid& g, const TsePre
         } else {
             for (int q = 0; q < 3; ++q) rec[q] = make_float2(0.0f, 0.0f);
         }
-        fz.K[col][6 * fz.Ncal + m] = rp;
+        *k_rp(fz.K[col], fz.ks, m) = rp;
+        *k_flag(fz.K[col], fz.ks, m) = f;
     }
     return pn * pn;
 }
@@ -258,7 +260,7 @@ int setup_pressure_dc(const TseGrid* grid, const TsePressureArgs* args, void* d_
     DcFuse fz;
     fz.K[0] = c.K[0];
     fz.K[1] = c.K[1];
-    fz.Ncal = c.Ncal;
+    fz.ks = c.ks;
     fz.partials = S.partials;
     fz.per_thread = (int)per;
     assemble_p_kernel<true><<<(unsigned)nb, kBlock, 0, stream>>>(*grid, *args, S.F, S.mask[0],

@@ -334,8 +334,8 @@ __device__ __forceinline__ void heat_terms(const TseGrid& g, const TseHeatArgs& 
 }
 
 // The exact form's per-cell arrays (TransportForm) and the flag byte.
-__device__ __forceinline__ void store_terms(const TransportForm& F, uint8_t* msk, const CellIdx& x,
-                                            const TransportTerms& T, int nx, int ny, int nz) {
+__device__ __forceinline__ uint8_t store_terms(const TransportForm& F, uint8_t* msk, const CellIdx& x,
+                                               const TransportTerms& T, int nx, int ny, int nz) {
     double* b = F.arr[x.col];
     const long long N = F.Ncal, m = x.m;
     const double omega = F.omega;
@@ -354,6 +354,7 @@ __device__ __forceinline__ void store_terms(const TransportForm& F, uint8_t* msk
     uint8_t f = neighbour_flags(x.i, x.j, x.k, nx, ny, nz);
     if (T.active) f |= F_ACTIVE;
     msk[m] = f;
+    return f;
 }
 
 __device__ __forceinline__ void store_padding(const TransportForm& F, uint8_t* msk, const CellIdx& x) {
@@ -366,9 +367,9 @@ __device__ __forceinline__ void store_padding(const TransportForm& F, uint8_t* m
 // omega co_q / Den, and r' with sum() of TransportForm, whose neighbour
 // products are the assembly's own co_q * Xn_q.
 __device__ __forceinline__ void store_dc(const TransportForm& F, const DcFuse& fz, const CellIdx& x,
-                                         const TransportTerms* T) {
+                                         const TransportTerms* T, uint8_t flags) {
     float* Kc = fz.K[x.col];
-    float2* rec = reinterpret_cast<float2*>(Kc + 6 * x.m);
+    float2* rec = k_rec(Kc, fz.ks, x.m);
     float rp = 0.0f;
     if (T && T->active) {
         const double omega = F.omega;
@@ -388,7 +389,8 @@ __device__ __forceinline__ void store_dc(const TransportForm& F, const DcFuse& f
 #pragma unroll
         for (int q = 0; q < 3; ++q) rec[q] = make_float2(0.0f, 0.0f);
     }
-    Kc[6 * fz.Ncal + x.m] = rp;
+    *k_rp(Kc, fz.ks, x.m) = rp;
+    *k_flag(Kc, fz.ks, x.m) = flags;
 }
 
 struct SpeciesKind {
@@ -452,14 +454,14 @@ __device__ __forceinline__ void assemble_body(const TseGrid& g, const typename K
         uint8_t* msk = x.col ? mask1 : mask0;
         if (x.pad) {
             store_padding(F, msk, x);
-            if (DC) store_dc(F, fz, x, nullptr);
+            if (DC) store_dc(F, fz, x, nullptr, 0);
             continue;
         }
         TransportTerms T;
         Kind::terms(g, a, x, L, faces, T);
-        store_terms(F, msk, x, T, L.nx, L.ny, L.nz);
+        const uint8_t f = store_terms(F, msk, x, T, L.nx, L.ny, L.nz);
         if (DC) {
-            store_dc(F, fz, x, &T);
+            store_dc(F, fz, x, &T, f);
             x2 = x2 + T.Xn * T.Xn;
         }
     }
@@ -595,7 +597,7 @@ static int setup_transport_dc(const TseGrid* grid, const Args* a, void* d_ws, si
     DcFuse fz;
     fz.K[0] = c.K[0];
     fz.K[1] = c.K[1];
-    fz.Ncal = c.Ncal;
+    fz.ks = c.ks;
     fz.partials = S.partials;
     fz.per_thread = (int)per;
     kernel<<<(unsigned)nb, kBlock, 0, stream>>>(*grid, *a, S.F, S.mask[0], S.mask[1], S.L, S.faces,
