@@ -135,3 +135,54 @@ def test_record_blocks_are_aligned_and_inside_their_array():
                 rec, rp, flag = base + 6 * o, base + 6 * C + o, 4 * (base + 7 * C) + o
                 assert rec * 4 % 8 == 0 and rec + 6 <= base + 6 * C
                 assert rp < base + 7 * C and flag < 4 * (base + block)
+
+
+@pytest.mark.parametrize("ring,groups", [(2, 1), (3, 1), (4, 1), (2, 2), (3, 2), (4, 2)])
+def test_parity_waits_never_pass_early(ring, groups):
+    """The stages of one pipeline: an in-order producer, copies that land in
+    any order, consumer groups that test a stage's full barrier by parity only.
+    A stage belongs to one group, so no group ever reads a use whose copies
+    have not landed and no barrier gets an arrival too many -- also over
+    phases whose chunk count is odd.  (With chunks dealt to the groups in turn
+    it happens within a few hundred tries; the second loop shows it.)"""
+    def run(by_stage, rng, phases=6, pmine=5):
+        total = phases * pmine
+        full = [0] * ring        # completed phases of each full barrier
+        empty = [0] * ring
+        issued, landing = 0, []
+        if by_stage:
+            mine = [[u for u in range(total) if (u % ring) % groups == g] for g in range(groups)]
+        else:
+            mine = [[u for u in range(total) if (u % pmine) % groups == g] for g in range(groups)]
+        at = [0] * groups
+        for _ in range(20000):
+            if all(at[g] == len(mine[g]) for g in range(groups)):
+                return True
+            what = rng.randrange(3)
+            if what == 0 and issued < total:
+                s = issued % ring
+                # mbarrier.try_wait.parity: true once the current phase's parity differs
+                if issued < ring or (empty[s] & 1) != ((issued // ring - 1) & 1):
+                    if issued >= ring and empty[s] != issued // ring:
+                        return False
+                    landing.append(issued)
+                    issued += 1
+            elif what == 1 and landing:
+                u = landing.pop(rng.randrange(len(landing)))
+                full[u % ring] += 1
+            elif what == 2:
+                g = rng.randrange(groups)
+                if at[g] < len(mine[g]):
+                    u = mine[g][at[g]]
+                    s = u % ring
+                    if (full[s] & 1) != ((u // ring) & 1):
+                        if full[s] != u // ring + 1:
+                            return False            # read before its copies landed
+                        empty[s] += 1
+                        at[g] += 1
+        return False
+
+    rng = random.Random(ring * 10 + groups)
+    assert all(run(True, rng) for _ in range(300))
+    if groups == 2 and ring == 4:
+        assert not all(run(False, rng) for _ in range(300))

@@ -316,12 +316,6 @@ __device__ __forceinline__ bool seg_wait(const unsigned* count, unsigned target,
     return true;
 }
 
-// A consumer warp has finished its chunks of one report.
-__device__ __forceinline__ void seg_arrive(uint64_t* bar) {
-    __syncwarp();
-    if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
-}
-
 template <int RING, int PIPES, int CHUNK, bool WIDE>
 __global__ void __launch_bounds__(DcLayout<PIPES, WIDE>::kThreads, DcLayout<PIPES, WIDE>::kMinBlocks)
     dc_sweep_tma_kernel(DcCtl c, TmaStage T) {
@@ -363,16 +357,15 @@ __global__ void __launch_bounds__(DcLayout<PIPES, WIDE>::kThreads, DcLayout<PIPE
     const int nseg = nch > (long long)first * nb ? 2 : 1;
     unsigned bars = 0;                           // device-wide barriers passed in this launch
     unsigned phases = 0;                         // colour phases before this one
-    // blocks with chunks of report s, and this block's warps there (a round is
-    // one consumer group's: 4 warps)
+    // blocks with chunks of report s, and the arrivals of this block's consumer
+    // warps there (one a warp and chunk)
     auto seg_blocks = [&](int s) {
         const long long rest = nch - (s ? (long long)first * nb : 0);
         return rest < (long long)nb ? (unsigned)rest : nb;
     };
-    auto seg_warps = [&](int s) {
+    auto seg_arrivals = [&](int s) {
         const long long n = s ? mine - first : mine < first ? mine : (long long)first;
-        const int groups = DcLayout<PIPES, WIDE>::kGroups;
-        return (unsigned)((n < groups ? (int)n : groups) * (kTmaGroup / 32));
+        return (unsigned)(n * (kTmaGroup / 32));
     };
     const bool leader = (b == 0 && tid == 0);
     const float sor = c.sor;
@@ -391,7 +384,7 @@ __global__ void __launch_bounds__(DcLayout<PIPES, WIDE>::kThreads, DcLayout<PIPE
             mbar_init(&empty[s], kTmaGroup / 32);   // one arrival per warp of a group
         }
         for (int s = 0; s < nseg; ++s) {
-            mbar_init(&seg_bar[s], seg_warps(s));
+            if (mine > (s ? first : 0)) mbar_init(&seg_bar[s], seg_arrivals(s));
             mbar_init(&gate[s], 1);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -455,14 +448,14 @@ __global__ void __launch_bounds__(DcLayout<PIPES, WIDE>::kThreads, DcLayout<PIPE
                     }
                 __syncwarp();
             } else {
-                bool cok = true;
-                int had = -1;   // the report this warp's last chunk belongs to
-                for (long long j = grank; j < pmine; j += kGroupsPerPipe) {
+                for (long long j = 0; j < pmine; ++j) {
                     const int i = pipe + (int)j * kPipes;
-                    const int now = i >= first;
-                    if (had >= 0 && now != had) seg_arrive(&seg_bar[had]);
-                    had = now;
                     const unsigned u = uses + (unsigned)j;
+                    // a stage belongs to one group for good: its parity waits
+                    // then see every use.  (By chunk, a group could ask for a
+                    // stage's next use while the other group's was still
+                    // arriving, and the parity would pass.)
+                    if ((int)((u % ring) % kGroupsPerPipe) != grank) continue;
                     const unsigned s = ring0 + u % ring;
                     const long long m0 = (b + (long long)i * nb) * C;
                     const int nval = (int)((Nc - m0) < C ? (Nc - m0) : C);
@@ -471,8 +464,7 @@ __global__ void __launch_bounds__(DcLayout<PIPES, WIDE>::kThreads, DcLayout<PIPE
                     // then every lane observes the completed phase (acquire)
                     int okw = 1;
                     if (lane == 0) okw = mbar_wait_flag(&full[s], (u / ring) & 1u, err);
-                    cok = __shfl_sync(0xffffffffu, okw, 0) != 0;
-                    if (!cok) break;
+                    if (!__shfl_sync(0xffffffffu, okw, 0)) break;
                     mbar_try_wait(&full[s], (u / ring) & 1u);
                     const unsigned char* stg = smem + (size_t)s * T.bytes;
                     // window offsets of cell l of the chunk (32-bit from here on)
@@ -510,10 +502,13 @@ __global__ void __launch_bounds__(DcLayout<PIPES, WIDE>::kThreads, DcLayout<PIPE
                         }
                     }
                     // the warp's reads of the stage are done: release it
+                    // and its stores belong to the phase's report
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&empty[s]);
+                    if (lane == 0) {
+                        mbar_arrive(&empty[s]);
+                        mbar_arrive(&seg_bar[i >= first]);
+                    }
                 }
-                if (cok && had >= 0) seg_arrive(&seg_bar[had]);
             }
             uses += (unsigned)pmine;
         }
