@@ -170,3 +170,50 @@ def test_sweep_variants_give_identical_results(cuda_device):
         assert numpy.array_equal(p[2], ref_p[2]), v
         assert (c[0], c[1], c[3], c[4]) == (ref_c[0], ref_c[1], ref_c[3], ref_c[4]), v
         assert numpy.array_equal(c[2], ref_c[2]), v
+
+
+# (more than 491,520 cells of a colour: the form that keeps the later cycles' words only;
+# the last but one has an odd number of cells of a colour, the last a padding cell each)
+@pytest.mark.parametrize("shape", [(17, 16, 24), (101, 99, 100), (3, 331, 1001), (701, 703, 1)])
+@pytest.mark.parametrize("omega", [1.0, 0.5, 0.0])
+def test_dc_transport_matches_the_exact_form(shape, omega, cuda_device):
+    """Species and heat solves against the FP64 kernels, with dispersivity in
+    some cells, zero and far out-of-range coefficients (the harmonic means'
+    general formula), the IMBLFLO term, several cycles, dt halvings and a stop
+    at min_dt."""
+    from transportse_b200 import workloads
+    rng = numpy.random.default_rng(sum(shape))
+    cfg = workloads.base_config("dct", *shape, *(rng.uniform(0.5, 2, n) for n in shape))
+    some = rng.uniform(size=shape) < 0.2
+    cfg.lf_l[:] = numpy.where(some, rng.uniform(0, 1, shape), 0.0)
+    cfg.lf_t[:] = numpy.where(some, rng.uniform(0, 0.3, shape), 0.0)
+    cfg.l_r[:] = rng.uniform(1.5, 3.5, shape)
+    cfg.rho_r[:], cfg.cp_r[:] = 2650.0, 900.0
+    cfg.C_IMBLFLO = cfg.T_IMBLFLO = True
+    one = numpy.ones(shape)
+    C, T = rng.uniform(0, 1, shape), rng.uniform(15, 80, shape)
+    phi, rho = rng.uniform(0.05, 0.3, shape), rng.uniform(995, 1150, shape)
+    D = [1e-6 * rng.uniform(0.5, 1.5, shape) for _ in range(3)]
+    for d, v in zip(D, (0.0, 1e-200, 1e-310)):
+        d[rng.uniform(size=shape) < 0.05] = v
+    l_f = 0.6 * one
+    l_f[rng.uniform(size=shape) < 0.05] = 0.0
+    B = (rng.uniform(size=shape) < 0.1).astype(float)
+    W = numpy.where(rng.uniform(size=shape) < 0.2, 1e-5, 0.0)
+    e = rng.uniform(-1e-6, 1e-6, shape)
+    q = [rng.uniform(-1e-4, 1e-4, shape) for _ in range(3)]
+    exact, dc = (NumpyKernels(model_for(cfg, cuda_device, p)) for p in ("fp64", "fp32dc"))
+
+    def species(nk, **kw):
+        return nk.compute_C(C.copy(), *D, phi, rho, *q, 600.0, B, W, one, e, C_conv=1e-11, **kw)
+
+    def heat(nk, **kw):
+        return nk.compute_T(T.copy(), l_f, 4180.0 * one, rho, phi, *q, 600.0, B, W, e, T_conv=1e-11, **kw)
+
+    for call in (species, heat):
+        for max_it, min_dt, cycle in ((100, 1e-8, 0), (100, 1e-8, 4), (6, 1e-8, 0), (3, 400.0, 0)):
+            kw = dict(omega=omega, SOR=1.1, max_it=max_it, inc_it=1.05, max_dt=1e5, min_dt=min_dt)
+            dc.m.dc_cycle = cycle
+            ro, rg = call(exact, **kw), call(dc, **kw)
+            assert rg[:2] == ro[:2] and rg[3] == ro[3], (call.__name__, max_it, rg[:2], ro[:2])
+            assert rel_err(rg[2], ro[2]) <= TOL, (call.__name__, max_it, rel_err(rg[2], ro[2]))

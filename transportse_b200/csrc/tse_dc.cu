@@ -32,6 +32,8 @@
 // L2 -- against 89 bytes of coefficients and flags for the FP64 form.
 //
 // Compiled with FMA contraction (no bit-exactness is claimed for this form).
+#include <type_traits>
+
 #include "tse_dc.cuh"
 #include "tse_dc_resident.cuh"
 
@@ -109,6 +111,66 @@ __global__ void __launch_bounds__(kBlock) dc_residual_kernel(Form F, DcCtl c) {
     const double o2 = residual_block_cells(F, c, blockIdx.x, gridDim.x);
     const double b = block_sum<kBlock>(o2, sh);
     if (threadIdx.x == 0) c.partials[blockIdx.x] = b;
+}
+
+// x += d and the residual of the new iterate in one pass, the new iterate into
+// another pair of arrays (Xn): neighbours' values are formed from their old
+// ones and their corrections.  The corrections are zeroed after the launch.
+// Bound: DRAM.  A thread takes two consecutive cells of a colour, and loads
+// everything before it computes, neighbours the grid does not have included
+// (inside the workspace and unused).  Cells of a colour: one thread each and
+// loads under their flags took 222 us at 256 x 256 x 128.
+template <class Form>
+__global__ void __launch_bounds__(kBlock) dc_apply_residual_kernel(Form F, DcCtl c, double* Xn0, double* Xn1) {
+    __shared__ double sh[kBlock / 32];
+    const long long Nc = c.L.Nc, N = c.Ncal, sx = c.L.SX, pairs = (Nc + 1) / 2;
+    const int h = c.L.H;
+    double o2 = 0.0;
+    for (long long t = (long long)blockIdx.x * kBlock + threadIdx.x; t < 2 * pairs;
+         t += (long long)gridDim.x * kBlock) {
+        const int col = t >= pairs;
+        const long long m = 2 * (t - (col ? pairs : 0));
+        const uint8_t* mk = (col ? c.mask[1] : c.mask[0]) + m;
+        const double* b = (col ? F.arr[1] : F.arr[0]) + m;
+        const double* Xo = (col ? c.X[0] : c.X[1]) + m;
+        const float* Do = (col ? c.D[0] : c.D[1]) + m;
+        // Ncal, the arrays' length, is a multiple of 32: a pair is inside
+        const uint8_t f0 = mk[0], f1 = mk[1];
+        double2 a[Form::kCoef];
+#pragma unroll
+        for (int k = 0; k < Form::kCoef; ++k)
+            if (F.later(k)) a[k] = *reinterpret_cast<const double2*>(b + k * N);
+        const double2 x = *reinterpret_cast<const double2*>((col ? c.X[1] : c.X[0]) + m);
+        const float2 d = *reinterpret_cast<const float2*>((col ? c.D[1] : c.D[0]) + m);
+        double xa[6], xb[6];
+        float da[6], db[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            const long long oa = nb_offset(q, sx, h, (long long)(f0 >> 7));
+            const long long ob = 1 + nb_offset(q, sx, h, (long long)(f1 >> 7));
+            xa[q] = Xo[oa];
+            da[q] = Do[oa];
+            xb[q] = Xo[ob];
+            db[q] = Do[ob];
+        }
+        const double x0 = (f0 & F_ACTIVE) ? x.x + (double)d.x : x.x;
+        const double x1 = (f1 & F_ACTIVE) ? x.y + (double)d.y : x.y;
+        float r0 = 0.0f, r1 = 0.0f;
+        if (f0 & F_ACTIVE) {
+            const double s = F.sum_with([&](int k) { return a[k].x; }, [&](int q) { return xa[q] + (double)da[q]; }, f0);
+            r0 = (float)((s - a[Form::kDen].x * x0) / a[Form::kDen].x);
+        }
+        if (f1 & F_ACTIVE) {
+            const double s = F.sum_with([&](int k) { return a[k].y; }, [&](int q) { return xb[q] + (double)db[q]; }, f1);
+            r1 = (float)((s - a[Form::kDen].y * x1) / a[Form::kDen].y);
+        }
+        *reinterpret_cast<double2*>((col ? Xn1 : Xn0) + m) = make_double2(x0, x1);
+        *reinterpret_cast<float2*>(k_rp(col ? c.K[1] : c.K[0], c.ks, m)) = make_float2(r0, r1);
+        o2 = o2 + x0 * x0;
+        if (m + 1 < Nc) o2 = o2 + x1 * x1;
+    }
+    const double s2 = block_sum<kBlock>(o2, sh);
+    if (threadIdx.x == 0) c.partials[blockIdx.x] = s2;
 }
 
 // x^2 total into the state; counts the cycle
@@ -714,11 +776,16 @@ static int dc_block_log2(const TseDcOptions* opts) {
     return opts && opts->chunk == 256 ? 8 : opts && opts->chunk == 1024 ? 10 : 9;
 }
 
-template <class Form>
+// A lean setup's dt halving assembles again: again(dt, nparts).
+struct NeverAgain {
+    int operator()(double, int*) const { return TSE_ERR_LAUNCH; }
+};
+template <class Form, class Again = NeverAgain>
 static int run_dc(SolveSetup<Form>& S, double dt, double inc_it, double max_dt, double min_dt,
                   double conv, int max_it, int pressure_schedule, int stop_on_first,
                   TseDcOptions* opts, double sor, int x_index, double* X_out,
-                  TseSolveStatus* d_status, cudaStream_t stream, int first_parts = 0) {
+                  TseSolveStatus* d_status, cudaStream_t stream, int first_parts,
+                  Again again = Again()) {
     const int cycle = opts ? opts->cycle : 0;
     const int cap = opts ? opts->max_blocks : 0;
     if (S.tail_bytes < dc_extra_bytes(S.L)) return TSE_ERR_WORKSPACE;
@@ -735,7 +802,7 @@ static int run_dc(SolveSetup<Form>& S, double dt, double inc_it, double max_dt, 
     c.sor = (float)sor;
     const bool timing = opts && opts->timing;
     // a grid that fits on the chip, and no staged variant asked for
-    if (!opts || (opts->chunk == 0 && opts->ring == 0 && opts->pipes == 0)) {
+    if (!S.lean && (!opts || (opts->chunk == 0 && opts->ring == 0 && opts->pipes == 0))) {
         const int rc = run_dc_resident(S, c, dt, cap, first_parts, X_out, d_status, timing ? opts : nullptr,
                                        stream);
         if (rc != 1) return rc;
@@ -778,12 +845,12 @@ static int run_dc(SolveSetup<Form>& S, double dt, double inc_it, double max_dt, 
     }
     const int nb = nb_tma > 0 ? nb_tma : sweep_blocks(S.L.Nc, cap);
     if (nb_tma > 0) sweep_head(S.L, nb_tma, T);
-    // first_parts > 0: the setup has written the records, r' and that many
-    // x^2 partials (the first cycle's scale and residual)
-    if (first_parts == 0) {
-        dc_scale_kernel<<<gcells, kBlock, 0, stream>>>(S.F, c);
-        if (cudaGetLastError() != cudaSuccess) return TSE_ERR_LAUNCH;
-    }
+    // the setup has written the records, r' and first_parts x^2 partials (the
+    // first cycle's scale and residual).  A lean setup's two iterates take
+    // turns, the later one in the arrays it leaves free.
+    constexpr int kAlt = std::is_same<Form, TransportForm>::value ? (int)TA_XN : 0;
+    double* alt[2] = {S.F.arr[0] + (size_t)kAlt * S.Ncal, S.F.arr[1] + (size_t)kAlt * S.Ncal};
+    double* const x0[2] = {c.X[0], c.X[1]};
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     if (timing) {
         opts->sweep_launches = 0;
@@ -845,6 +912,30 @@ static int run_dc(SolveSetup<Form>& S, double dt, double inc_it, double max_dt, 
             opts->sweep_ms += ms;
         }
         prev_it = head[1];
+        if (S.lean && event == EV_STOP_HALVED) {
+            // the caller's field still holds the entry state
+            dc_status_kernel<<<1, 1, 0, stream>>>(c.st, d_status);
+            if (timing) {
+                cudaEventDestroy(ev0);
+                cudaEventDestroy(ev1);
+            }
+            return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
+        }
+        if (S.lean && event == EV_HALVE) {
+            double half = 0.0;
+            if (cudaMemcpyAsync(&half, &c.st->dt, sizeof(double), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+                cudaStreamSynchronize(stream) != cudaSuccess ||
+                cudaMemsetAsync(dbase, 0, (size_t)2 * dlen * sizeof(float), stream) != cudaSuccess ||
+                again(half, &first_parts) != TSE_OK) {
+                rc = TSE_ERR_LAUNCH;
+                break;
+            }
+            if (c.X[0] != x0[0]) {
+                std::swap(c.X[0], alt[0]);
+                std::swap(c.X[1], alt[1]);
+            }
+            continue;
+        }
         if (event == EV_HALVE || event == EV_STOP_HALVED) {
             dc_halve_kernel<<<gcells, kBlock, 0, stream>>>(S.F, c);
             if (cudaGetLastError() != cudaSuccess) { rc = TSE_ERR_LAUNCH; break; }
@@ -855,6 +946,20 @@ static int run_dc(SolveSetup<Form>& S, double dt, double inc_it, double max_dt, 
         if (event == EV_CONVERGED || event == EV_STOP) {
             final_apply = true;   // x += d fused with the unpack below
             break;
+        }
+        if (S.lean) {
+            const int rb = res_blocks(S.L.Nc);
+            if constexpr (std::is_same<Form, TransportForm>::value)
+                dc_apply_residual_kernel<<<(unsigned)rb, kBlock, 0, stream>>>(S.F, c, alt[0], alt[1]);
+            std::swap(c.X[0], alt[0]);
+            std::swap(c.X[1], alt[1]);
+            first_parts = rb;
+            if (cudaMemsetAsync(dbase, 0, (size_t)2 * dlen * sizeof(float), stream) != cudaSuccess ||
+                cudaGetLastError() != cudaSuccess) {
+                rc = TSE_ERR_LAUNCH;
+                break;
+            }
+            continue;
         }
         dc_apply_kernel<<<gcells, kBlock, 0, stream>>>(c);
         if (cudaGetLastError() != cudaSuccess) { rc = TSE_ERR_LAUNCH; break; }
@@ -940,6 +1045,11 @@ template int dc_halve<TransportForm>(const TransportForm&, const DcCtl&, cudaStr
 
 using namespace tse;
 
+// transport solves too large to be resident keep the later cycles' words only
+static bool lean_grid(const TseGrid* grid) {
+    return make_layout(grid->nx, grid->ny, grid->nz).Nc > kDcResMaxNc;
+}
+
 extern "C" int32_t tse_compute_P_dc(const TseGrid* grid, const TsePressureArgs* args,
                                     TseDcOptions* opts,
                                     TseSolveStatus* d_status, void* d_ws, size_t ws_bytes,
@@ -971,11 +1081,17 @@ extern "C" int32_t tse_compute_C_dc(const TseGrid* grid, const TseSpeciesArgs* a
     cudaStream_t stream = (cudaStream_t)stream_;
     TransportSetup S;
     S.ks = dc_block_log2(opts);
+    S.lean = lean_grid(grid);
     int nparts = 0;
     int rc = setup_species_dc(grid, a, d_ws, ws_bytes, stream, S, &nparts);
     if (rc != TSE_OK) return rc;
+    auto again = [&](double dt, int* np) {
+        TseSpeciesArgs half = *a;
+        half.dt = dt;
+        return again_species_dc(grid, &half, stream, S, np);
+    };
     return run_dc(S, a->dt, a->inc_it, a->max_dt, a->min_dt, a->conv, a->max_it, 0,
-                  a->omega == 0.0, opts, a->SOR, TA_X, a->C, d_status, stream, nparts);
+                  a->omega == 0.0, opts, a->SOR, TA_X, a->C, d_status, stream, nparts, again);
 }
 
 extern "C" int32_t tse_compute_T_dc(const TseGrid* grid, const TseHeatArgs* a,
@@ -990,9 +1106,15 @@ extern "C" int32_t tse_compute_T_dc(const TseGrid* grid, const TseHeatArgs* a,
     cudaStream_t stream = (cudaStream_t)stream_;
     TransportSetup S;
     S.ks = dc_block_log2(opts);
+    S.lean = lean_grid(grid);
     int nparts = 0;
     int rc = setup_heat_dc(grid, a, d_ws, ws_bytes, stream, S, &nparts);
     if (rc != TSE_OK) return rc;
+    auto again = [&](double dt, int* np) {
+        TseHeatArgs half = *a;
+        half.dt = dt;
+        return again_heat_dc(grid, &half, stream, S, np);
+    };
     return run_dc(S, a->dt, a->inc_it, a->max_dt, a->min_dt, a->conv, a->max_it, 0,
-                  a->omega == 0.0, opts, a->SOR, TA_X, a->T, d_status, stream, nparts);
+                  a->omega == 0.0, opts, a->SOR, TA_X, a->T, d_status, stream, nparts, again);
 }

@@ -233,6 +233,12 @@ int setup_species_dc(const TseGrid* grid, const TseSpeciesArgs* a, void* d_ws, s
 int setup_heat_dc(const TseGrid* grid, const TseHeatArgs* a, void* d_ws, size_t ws_bytes,
                   cudaStream_t stream, TransportSetup& S, int* nparts);
 
+// the same assembly again (a lean setup's dt halving: a->dt is the new one)
+int again_species_dc(const TseGrid* grid, const TseSpeciesArgs* a, cudaStream_t stream, TransportSetup& S,
+                     int* nparts);
+int again_heat_dc(const TseGrid* grid, const TseHeatArgs* a, cudaStream_t stream, TransportSetup& S,
+                  int* nparts);
+
 // Fill a control record for a solve whose exact-form setup is S (the FP32
 // arrays live in S.tail); returns the first byte after the FP32 arrays.
 template <class Form>

@@ -139,6 +139,7 @@ struct TransportForm {
     long long Ncal, SX;
     int H;
     int useY, useEX;
+    int useW;   // 0: the lean mixed-precision form, whose RXN holds every fixed term
     double omega, SOR;
 
     // numerator of the update (tse.py:870-874), in the reference's order;
@@ -154,7 +155,7 @@ struct TransportForm {
         double num = omega * s;
         if (useY) num = num + a(TA_Y);
         num = num + a(TA_RXN);
-        num = num + a(TA_W);
+        if (useW) num = num + a(TA_W);
         num = num - (useEX ? a(TA_EX) : 0.0);
         return num;
     }
@@ -188,6 +189,8 @@ struct TransportForm {
              : k == TA_EX ? (G2 ? k - !G1 : -1)
                           : k - !G1 - !G2;
     }
+    // does a lean solve's sum() or update read array k?
+    __device__ __forceinline__ bool later(int k) const { return k <= TA_F || k == TA_RXN || k == TA_DEN; }
     bool res_g1() const { return useY != 0; }
     bool res_g2() const { return useEX != 0; }
     template <bool G1, bool G2>
@@ -195,6 +198,7 @@ struct TransportForm {
         TransportForm f = *this;
         f.useY = G1;
         f.useEX = G2;
+        f.useW = 1;
         return f;
     }
     static constexpr int kArrays = TA_COUNT;
@@ -241,6 +245,9 @@ struct SolveSetup {
     char* tail;          // workspace bytes after the exact form's arrays
     size_t tail_bytes;
     double* faces = nullptr;   // transport: the face pass's values
+    // transport, mixed precision: the later cycles' nine words only (a dt
+    // halving assembles again); set by a caller that can do so
+    bool lean = false;
     int ks = 9;          // mixed-precision form: log2 of the record blocks' cells
 };
 using PressureSetup = SolveSetup<PressureForm>;

@@ -9,6 +9,8 @@
 //   X = (1-SOR) X + SOR (omega (Mnew+Nnew+Onew+Pnew+Qnew+Rnew)
 //                        + (1-omega) (...) + R Xn + W - E) / (R - omega M)
 // (tse.py:870-875, 1038-1043) term by term.  Compiled with --fmad=false.
+#include <algorithm>
+
 #include "tse_dc.cuh"
 #include "tse_forms.cuh"
 #include "tse_rbsolve.cuh"
@@ -251,11 +253,11 @@ __device__ __forceinline__ AxisTerms heat_axis(const double* __restrict__ K1, co
 }
 
 // The per-cell terms of a transport solve: the six neighbour coefficients
-// (x+, x-, y+, y-, z+, z-), M, (1-omega)-part Mo, R and its numerator, source,
-// IMBLFLO term and the neighbour sum of the initial iterate in sum()'s order.
+// (x+, x-, y+, y-, z+, z-), M, (1-omega)-part Mo, R and its numerator, source
+// and IMBLFLO term.
 struct TransportTerms {
     double co[6];
-    double s, Mo, Xn, Rnum, R, M, W, EX;
+    double Mo, Xn, Rnum, R, M, W, EX;
     bool active;
 };
 
@@ -272,13 +274,6 @@ __device__ __forceinline__ void combine_axes(const AxisTerms& X, const AxisTerms
           Z.maxP;
     T.Xn = Xn;
     T.Mo = Xn * T.M + X.oldP + X.oldM + Y.oldP + Y.oldM + Z.oldP + Z.oldM;
-    double s = X.oldP;
-    s = s + X.oldM;
-    s = s + Y.oldP;
-    s = s + Y.oldM;
-    s = s + Z.oldP;
-    s = s + Z.oldM;
-    T.s = s;
 }
 
 // coefficient part of compute_C.solve (tse.py:795-868)
@@ -334,8 +329,8 @@ __device__ __forceinline__ void heat_terms(const TseGrid& g, const TseHeatArgs& 
 }
 
 // The exact form's per-cell arrays (TransportForm) and the flag byte.
-__device__ __forceinline__ uint8_t store_terms(const TransportForm& F, uint8_t* msk, const CellIdx& x,
-                                               const TransportTerms& T, int nx, int ny, int nz) {
+__device__ __forceinline__ void store_terms(const TransportForm& F, uint8_t* msk, const CellIdx& x,
+                                            const TransportTerms& T, int nx, int ny, int nz) {
     double* b = F.arr[x.col];
     const long long N = F.Ncal, m = x.m;
     const double omega = F.omega;
@@ -354,43 +349,12 @@ __device__ __forceinline__ uint8_t store_terms(const TransportForm& F, uint8_t* 
     uint8_t f = neighbour_flags(x.i, x.j, x.k, nx, ny, nz);
     if (T.active) f |= F_ACTIVE;
     msk[m] = f;
-    return f;
 }
 
 __device__ __forceinline__ void store_padding(const TransportForm& F, uint8_t* msk, const CellIdx& x) {
     double* b = F.arr[x.col];
     for (int q = 0; q < TA_COUNT; ++q) b[q * F.Ncal + x.m] = 0.0;
     msk[x.m] = 0;
-}
-
-// The first correction cycle of the mixed-precision form (DcFuse): K'_q =
-// omega co_q / Den, and r' with sum() of TransportForm, whose neighbour
-// products are the assembly's own co_q * Xn_q.
-__device__ __forceinline__ void store_dc(const TransportForm& F, const DcFuse& fz, const CellIdx& x,
-                                         const TransportTerms* T, uint8_t flags) {
-    float* Kc = fz.K[x.col];
-    float2* rec = k_rec(Kc, fz.ks, x.m);
-    float rp = 0.0f;
-    if (T && T->active) {
-        const double omega = F.omega;
-        const double den = T->R - omega * T->M;
-        const double rden = 1.0 / den;
-#pragma unroll
-        for (int q = 0; q < 3; ++q)
-            rec[q] = make_float2((float)(omega * T->co[2 * q] * rden),
-                                 (float)(omega * T->co[2 * q + 1] * rden));
-        double num = omega * T->s;
-        if (F.useY) num = num + (1 - omega) * T->Mo;
-        num = num + T->R * T->Xn;
-        num = num + T->W;
-        num = num - (F.useEX ? T->EX : 0.0);
-        rp = (float)((num - den * T->Xn) * rden);
-    } else {
-#pragma unroll
-        for (int q = 0; q < 3; ++q) rec[q] = make_float2(0.0f, 0.0f);
-    }
-    *k_rp(Kc, fz.ks, x.m) = rp;
-    *k_flag(Kc, fz.ks, x.m) = flags;
 }
 
 struct SpeciesKind {
@@ -437,54 +401,311 @@ struct HeatKind {
 #endif
 constexpr int kAssembleMinBlocks = TSE_ASM_MINB;
 
-// One thread per cell of the padded natural order (DC: per_thread
-// consecutive blocks of kBlock cells each, so the x^2 partials stay few).
-template <class Kind, bool DC>
+// One thread per cell of the padded natural order.
+template <class Kind>
 __device__ __forceinline__ void assemble_body(const TseGrid& g, const typename Kind::Args& a,
-                                              const TransportForm& F, uint8_t* mask0,
-                                              uint8_t* mask1, const Layout& L,
-                                              const double* __restrict__ faces, const DcFuse& fz) {
-    __shared__ double sh[kBlock / 32];
-    double x2 = 0.0;
-    const int per = DC ? fz.per_thread : 1;
-    for (int s = 0; s < per; ++s) {
-        CellIdx x;
-        const long long t = ((long long)blockIdx.x * per + s) * kBlock + threadIdx.x;
-        if (!decode_padded(t, L, x)) break;
-        uint8_t* msk = x.col ? mask1 : mask0;
-        if (x.pad) {
-            store_padding(F, msk, x);
-            if (DC) store_dc(F, fz, x, nullptr, 0);
-            continue;
-        }
-        TransportTerms T;
-        Kind::terms(g, a, x, L, faces, T);
-        const uint8_t f = store_terms(F, msk, x, T, L.nx, L.ny, L.nz);
-        if (DC) {
-            store_dc(F, fz, x, &T, f);
-            x2 = x2 + T.Xn * T.Xn;
-        }
+                                              const TransportForm& F, uint8_t* mask0, uint8_t* mask1,
+                                              const Layout& L, const double* __restrict__ faces) {
+    CellIdx x;
+    if (!decode_padded((long long)blockIdx.x * kBlock + threadIdx.x, L, x)) return;
+    uint8_t* msk = x.col ? mask1 : mask0;
+    if (x.pad) {
+        store_padding(F, msk, x);
+        return;
     }
-    if (DC) {
-        const double b = block_sum<kBlock>(x2, sh);
-        if (threadIdx.x == 0) fz.partials[blockIdx.x] = b;
-    }
+    TransportTerms T;
+    Kind::terms(g, a, x, L, faces, T);
+    store_terms(F, msk, x, T, L.nx, L.ny, L.nz);
 }
 
 // coefficient part of compute_C.solve (tse.py:795-868)
-template <bool DC>
 __global__ void __launch_bounds__(kBlock, kAssembleMinBlocks)
-    assemble_c_kernel(TseGrid g, TseSpeciesArgs a, TransportForm F, uint8_t* mask0, uint8_t* mask1,
-                      Layout L, const double* faces, DcFuse fz) {
-    assemble_body<SpeciesKind, DC>(g, a, F, mask0, mask1, L, faces, fz);
+    assemble_c_kernel(TseGrid g, TseSpeciesArgs a, TransportForm F, uint8_t* mask0, uint8_t* mask1, Layout L,
+                      const double* faces) {
+    assemble_body<SpeciesKind>(g, a, F, mask0, mask1, L, faces);
 }
 
 // coefficient part of compute_T.solve (tse.py:930-1036)
-template <bool DC>
 __global__ void __launch_bounds__(kBlock, kAssembleMinBlocks)
-    assemble_t_kernel(TseGrid g, TseHeatArgs a, TransportForm F, uint8_t* mask0, uint8_t* mask1,
-                      Layout L, const double* faces, DcFuse fz) {
-    assemble_body<HeatKind, DC>(g, a, F, mask0, mask1, L, faces, fz);
+    assemble_t_kernel(TseGrid g, TseHeatArgs a, TransportForm F, uint8_t* mask0, uint8_t* mask1, Layout L,
+                      const double* faces) {
+    assemble_body<HeatKind>(g, a, F, mask0, mask1, L, faces);
+}
+
+// ---------------------------------------------- the mixed-precision assembly
+// One pass from the inputs to the first correction cycle (DcFuse): records
+// K'_q = omega co_q / Den, r' of the initial iterate, flags, x^2 partials, and
+// the FP64 arrays later cycles read.  The same terms as the exact form's, with
+// each cell forming its own six faces' means: a face pass's 24 or 48 bytes a
+// cell to write and read again cost more than the means.
+//
+// What bounded it were instructions, FP64 divisions above all (an SM finishes
+// 3.7 a clock against 63 additions, and each is some 20 instructions), then the
+// latency of its loads, then its 15 stored arrays.  So:
+//  - quotients by a spacing, by a product or sum of two spacings or by dt take
+//    the divisor's reciprocal from a table {b, 1 / b} (axis_tables_kernel) and
+//    one correction step with fused operations, q = a r, q + r (a - b q) (the
+//    closing step of a division by Newton's method, Markstein 1990): the
+//    rounded quotient but for rare cases one unit in the last place off;
+//  - a harmonic mean is (d1 + d2) H1 H2 / (d1 H2 + d2 H1), one division, and
+//    heat's two products of means share one each;
+//  - with `lean` (a solve that streams its grid and runs alone) the terms only
+//    later cycles' sums need are stored, nine words instead of fifteen; a dt
+//    halving runs this pass again.
+__device__ __forceinline__ double qdiv(double a, double2 b) {
+    const double q = a * b.y;
+    const double r = __fma_rn(__fma_rn(-b.x, q, a), b.y, q);
+    return (__double2hiint(q) & 0x7ff00000) == 0x7ff00000 ? q : r;   // inf, NaN
+}
+// |v| far from both ends of the exponent range (and not 0, inf or NaN)
+__device__ __forceinline__ bool mid_range(double v) {
+    const unsigned e = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu;
+    return e - 64u < 1920u;
+}
+
+// Per axis and index i four pairs {b, 1 / b}: b = d[i], the + face's and the -
+// face's (0.5 (d[i] + d[i +- 1])) d[i], and d[i] + d[i + 1] ({1, 1} where the
+// axis has no such neighbour); all indices' first pairs (x, y, z axes in turn),
+// then all second pairs ...: along z a warp's loads are contiguous.
+constexpr int kTabPairs = 4;
+__global__ void axis_tables_kernel(TseGrid g, double2* tab) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= g.nx + g.ny + g.nz) return;
+    double2* t = tab + i;
+    const int st = g.nx + g.ny + g.nz;
+    const double* d = g.dx;
+    int n = g.nx;
+    if (i >= g.nx + g.ny) {
+        i -= g.nx + g.ny;
+        d = g.dz;
+        n = g.nz;
+    } else if (i >= g.nx) {
+        i -= g.nx;
+        d = g.dy;
+        n = g.ny;
+    }
+    const double dd = d[i];
+    double b[kTabPairs] = {dd, 1.0, 1.0, 1.0};
+    if (i + 1 < n) {
+        b[1] = (0.5 * (d[i + 1] + dd)) * dd;
+        b[3] = d[i + 1] + dd;
+    }
+    if (i > 0) b[2] = (0.5 * (d[i - 1] + dd)) * dd;
+    for (int q = 0; q < kTabPairs; ++q) t[q * st] = make_double2(b[q], 1.0 / b[q]);
+}
+static size_t axis_table_bytes(const Layout& L) {
+    return align256((size_t)(L.nx + L.ny + L.nz) * kTabPairs * sizeof(double2));
+}
+
+// the dispersion terms as a call: cells without dispersivity leave its
+// registers to the rest of the pass
+__device__ __noinline__ void dispersivity_call(const double* qx, const double* qy, const double* qz,
+                                               const double* l_l, const double* l_t, const double* B, int i,
+                                               int j, int k, int nx, int ny, int nz, double* D) {
+    dispersivity_dev(qx, qy, qz, l_l, l_t, B, i, j, k, nx, ny, nz, D);
+}
+
+// axis(): one axis of a cell, added to M, to the neighbour sum s of the initial
+// iterate and into the two coefficients.  A face is always formed with its +
+// cell's values first, so both its cells get the same bits.
+struct SpeciesFast {
+    using Args = TseSpeciesArgs;
+    static constexpr int kBlocks = 5;   // resident on a SM
+    static __device__ __forceinline__ const double* X(const Args& a) { return a.C; }
+    static __device__ __forceinline__ const double* B(const Args& a) { return a.BC; }
+    static __device__ __forceinline__ const double* W(const Args& a) { return a.WC; }
+    static __device__ __forceinline__ const double* field(const Args& a, int axis) {
+        return axis == 0 ? a.D_fx : axis == 1 ? a.D_fy : a.D_fz;
+    }
+    // harm2(D) amean2(phi) of the face between cells p (+) and m (-)
+    static __device__ __forceinline__ double mean(const double* D, const double* phi, long long p, long long m,
+                                                  double dp, double dm, double2 s) {
+        const double H1 = D[p], H2 = D[m];
+        const double por = qdiv(phi[p] * dp + phi[m] * dm, s);
+        if (!(H1 != 0.0 && H2 != 0.0)) return 0.0 * por;
+        const double n = s.x * (H1 * H2), t = __fma_rn(dp, H2, dm * H1);
+        if (mid_range(H1 * H2) && mid_range(n) && mid_range(t)) return n / t * por;
+        return (dp + dm) / (dp / H1 + dm / H2) * por;
+    }
+    static __device__ __forceinline__ void axis(const Args& a, int ax, const double* q, const double2* t,
+                                                int ts, long long c, long long st, bool hp, bool hm, double DdP,
+                                                double DdM, double& M, double& s, double& coP, double& coM) {
+        const double* D = field(a, ax);
+        const double2 b = t[0];
+        const double z = 0.0 * b.y;
+        coP = coM = 0.0;
+        if (hp) {
+            const double qc = q[c];
+            const double f = mean(D, a.phi, c + st, c, t[1].x, b.x, t[3 * ts]);
+            const double d = qdiv(f + DdP, t[ts]), qd = qdiv(qc, b);
+            coP = d - ((0.0 < qc) ? z : qd);
+            M = M - d - ((0.0 > qc) ? z : qd);
+            s = s + coP * a.C[c + st];
+        }
+        if (hm) {
+            const double qm = q[c - st];
+            const double f = mean(D, a.phi, c, c - st, b.x, t[-1].x, t[3 * ts - 1]);
+            const double d = qdiv(f + DdM, t[2 * ts]), qd = qdiv(qm, b);
+            coM = d + ((0.0 > qm) ? z : qd);
+            M = M - d + ((0.0 < qm) ? z : qd);
+            s = s + coM * a.C[c - st];
+        }
+    }
+    static __device__ __forceinline__ void rest(const Args& a, long long c, double Xn, double& Rnum, double& EX) {
+        Rnum = a.RC[c] * a.phi[c];
+        EX = a.imblflo ? Xn / a.rho_f[c] * a.e[c] : 0.0;
+    }
+};
+struct HeatFast {
+    using Args = TseHeatArgs;
+    static constexpr int kBlocks = 4;
+    static __device__ __forceinline__ const double* X(const Args& a) { return a.T; }
+    static __device__ __forceinline__ const double* B(const Args& a) { return a.BT; }
+    static __device__ __forceinline__ const double* W(const Args& a) { return a.WT; }
+    // the conductivity mix and the mean of rho_f times that of cp_f
+    static __device__ __forceinline__ void means(const Args& a, long long p, long long m, double dp, double dm,
+                                                 double2 s, double& k1, double& rc) {
+        const double por = qdiv(a.phi[p] * dp + a.phi[m] * dm, s);
+        const double f1 = a.l_f[p], f2 = a.l_f[m], r1 = a.l_r[p], r2 = a.l_r[m];
+        const double c1 = a.cp_f[p], c2 = a.cp_f[m], h1 = a.rho_f[p], h2 = a.rho_f[m];
+        // numerators and denominators of the four harmonic means, less the
+        // common factor dp + dm
+        const double nf = f1 * f2, tf = __fma_rn(dp, f2, dm * f1), nr = r1 * r2, tr = __fma_rn(dp, r2, dm * r1);
+        const double nc = c1 * c2, tc = __fma_rn(dp, c2, dm * c1), nh = h1 * h2, th = __fma_rn(dp, h2, dm * h1);
+        const double nk = s.x * __fma_rn((1 - por) * nr, tf, por * nf * tr), tk = tf * tr;
+        const double n2 = (s.x * nc) * (s.x * nh), t2 = tc * th;
+        if (mid_range(nf) && mid_range(nr) && mid_range(nc) && mid_range(nh) && mid_range(tk) &&
+            mid_range(t2) && mid_range(nk) && mid_range(n2)) {
+            k1 = nk / tk;
+            rc = n2 / t2;
+        } else {
+            rc = harm2(h1, h2, dp, dm) * harm2(c1, c2, dp, dm);
+            k1 = (1 - por) * harm2(r1, r2, dp, dm) + por * harm2(f1, f2, dp, dm);
+        }
+    }
+    static __device__ __forceinline__ void axis(const Args& a, int, const double* q, const double2* t, int ts,
+                                                long long c, long long st, bool hp, bool hm, double DdP,
+                                                double DdM, double& M, double& s, double& coP, double& coM) {
+        const double2 b = t[0];
+        coP = coM = 0.0;
+        if (hp) {
+            const double qc = q[c];
+            double k1, rc;
+            means(a, c + st, c, t[1].x, b.x, t[3 * ts], k1, rc);
+            const double d = qdiv(k1 + DdP * rc, t[ts]), S = qdiv(rc, b);
+            coP = d - min0(qc) * S;
+            M = M - d - max0(qc) * S;
+            s = s + coP * a.T[c + st];
+        }
+        if (hm) {
+            const double qm = q[c - st];
+            double k1, rc;
+            means(a, c, c - st, b.x, t[-1].x, t[3 * ts - 1], k1, rc);
+            const double d = qdiv(k1 + DdM * rc, t[2 * ts]), S = qdiv(rc, b);
+            coM = d + max0(qm) * S;
+            M = M - d + min0(qm) * S;
+            s = s + coM * a.T[c - st];
+        }
+    }
+    static __device__ __forceinline__ void rest(const Args& a, long long c, double Xn, double& Rnum, double& EX) {
+        const double por = a.phi[c];
+        Rnum = por * a.rho_f[c] * a.cp_f[c] + (1 - por) * a.rho_r[c] * a.cp_r[c];
+        EX = a.imblflo ? a.cp_f[c] * Xn * a.e[c] : 0.0;
+    }
+};
+
+// Measured at 256 x 256 x 128 (B200), dispersivity 0, with the first cycle's
+// records: species 582 us (face pass and assembly took 963), heat 747 (1089).
+// It waits for its loads most of the time (1.7 of 4 instructions a clock): more
+// blocks a SM help as long as registers last (species 630 us with 4 blocks, heat
+// 858 with 5), loads gathered ahead of the arithmetic cost more registers than
+// they hide (species 640 and more).
+template <class Kind, bool LEAN>
+__global__ void __launch_bounds__(kBlock, Kind::kBlocks)
+    assemble_fast_kernel(TseGrid g, typename Kind::Args a, TransportForm F, uint8_t* mask0, uint8_t* mask1,
+                         Layout L, const double2* __restrict__ tab, DcFuse fz) {
+    __shared__ double sh[kBlock / 32];
+    const double2 dt = make_double2(a.dt, 1.0 / a.dt);
+    const double omega = F.omega;
+    const long long N = F.Ncal;
+    const int ts = L.nx + L.ny + L.nz;
+    double x2 = 0.0;
+    for (int rep = 0; rep < fz.per_thread; ++rep) {
+        CellIdx x;
+        const long long t = ((long long)blockIdx.x * fz.per_thread + rep) * kBlock + threadIdx.x;
+        if (!decode_padded(t, L, x)) break;
+        uint8_t* msk = x.col ? mask1 : mask0;
+        double* b = (x.col ? F.arr[1] : F.arr[0]) + x.m;
+        float* Kc = x.col ? fz.K[1] : fz.K[0];
+        float2* rec = k_rec(Kc, fz.ks, x.m);
+        if (x.pad) {
+            for (int q = 0; q < TA_COUNT; ++q) b[q * N] = 0.0;
+            msk[x.m] = 0;
+            for (int q = 0; q < 3; ++q) rec[q] = make_float2(0.0f, 0.0f);
+            *k_rp(Kc, fz.ks, x.m) = 0.0f;
+            *k_flag(Kc, fz.ks, x.m) = 0;
+            continue;
+        }
+        const int i = x.i, j = x.j, k = x.k;
+        const long long c = x.c;
+        double Dd[6] = {0, 0, 0, 0, 0, 0};
+        if (a.l_l[c] != 0 || a.l_t[c] != 0)
+            dispersivity_call(a.qx, a.qy, a.qz, a.l_l, a.l_t, Kind::B(a), i, j, k, L.nx, L.ny, L.nz, Dd);
+        double M = 0.0, s = 0.0, co[6];
+        Kind::axis(a, 0, a.qx, tab + i, ts, c, (long long)L.ny * L.nz, i != L.nx - 1, i != 0, Dd[3],
+                   Dd[0], M, s, co[0], co[1]);
+        Kind::axis(a, 1, a.qy, tab + L.nx + j, ts, c, L.nz, j != L.ny - 1, j != 0, Dd[4], Dd[1], M, s,
+                   co[2], co[3]);
+        Kind::axis(a, 2, a.qz, tab + L.nx + L.ny + k, ts, c, 1, k != L.nz - 1, k != 0, Dd[5], Dd[2], M,
+                   s, co[4], co[5]);
+        const double Xn = Kind::X(a)[c], W = Kind::W(a)[c];
+        const bool active = !(Kind::B(a)[c] != 0.0);
+        double Rnum, EX;
+        Kind::rest(a, c, Xn, Rnum, EX);
+        const double R = qdiv(Rnum, dt), den = R - omega * M;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) b[q * N] = co[q];
+        // the terms that stay fixed during the solve, in sum()'s order
+        double num = omega * s, fix;
+        const double Y = F.useY ? (1 - omega) * (Xn * M + s) : 0.0;
+        fix = R * Xn;
+        if (F.useY) fix = Y + fix;
+        fix = fix + W;
+        if (F.useEX) fix = fix - EX;
+        num = num + fix;
+        b[TA_DEN * N] = den;
+        b[TA_X * N] = Xn;
+        if (LEAN) {
+            b[TA_RXN * N] = fix;
+        } else {
+            b[TA_RXN * N] = R * Xn;
+            b[TA_W * N] = W;
+            if (F.useY) b[TA_Y * N] = Y;
+            if (F.useEX) b[TA_EX * N] = EX;
+            b[TA_RNUM * N] = Rnum;
+            b[TA_M * N] = M;
+            b[TA_XN * N] = Xn;
+        }
+        uint8_t f = neighbour_flags(i, j, k, L.nx, L.ny, L.nz);
+        if (active) f |= F_ACTIVE;
+        msk[x.m] = f;
+        *k_flag(Kc, fz.ks, x.m) = f;
+        float rp = 0.0f;
+        if (active) {
+            const double rden = 1.0 / den, w = omega * rden;
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+                rec[q] = make_float2((float)(co[2 * q] * w), (float)(co[2 * q + 1] * w));
+            rp = (float)((num - den * Xn) * rden);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) rec[q] = make_float2(0.0f, 0.0f);
+        }
+        *k_rp(Kc, fz.ks, x.m) = rp;
+        x2 = x2 + Xn * Xn;
+    }
+    const double bs = block_sum<kBlock>(x2, sh);
+    if (threadIdx.x == 0) fz.partials[blockIdx.x] = bs;
 }
 
 // the face pass before an assembly: one thread per cell, natural order
@@ -520,7 +741,8 @@ size_t transport_ws_bytes(const Layout& L, long long* Ncal_out) {
     b += align256((size_t)2 * kMaxBlocks * sizeof(double));
     b += 2 * align256((size_t)Ncal);
     b += 2 * (size_t)TA_COUNT * Ncal * sizeof(double);
-    b += align256((size_t)kTransportFaceWords * L.nx * L.ny * L.nz * sizeof(double));   // face pass
+    // the exact form's face pass, or the mixed-precision form's axis tables
+    b += std::max(align256((size_t)kTransportFaceWords * L.nx * L.ny * L.nz * sizeof(double)), axis_table_bytes(L));
     return b;
 }
 
@@ -551,14 +773,14 @@ static int carve_transport(const TseGrid* grid, const Args* a, void* d_ws, size_
     S.F.SOR = a->SOR;
     S.F.useY = a->omega != 1.0;
     S.F.useEX = imbl != 0;
+    S.F.useW = 1;
     S.tail = (char*)d_ws + need;
     S.tail_bytes = ws_bytes - need;
     if (cudaMemsetAsync(S.bar, 0, sizeof(GridBarrier), stream) != cudaSuccess) return TSE_ERR_LAUNCH;
     return TSE_OK;
 }
 
-// carve + the exact form's assembly
-// the face pass of a transport setup
+// the face pass of an exact setup
 template <class Args, class FacesK>
 static void launch_faces(const TseGrid* grid, const Args* a, const TransportSetup& S, FacesK fk,
                          cudaStream_t stream) {
@@ -576,20 +798,14 @@ static int setup_transport(const TseGrid* grid, const Args* a, void* d_ws, size_
     launch_faces(grid, a, S, fk, stream);
     const long long total = (long long)S.L.nx * S.L.ny * S.L.nzp;
     kernel<<<(unsigned)((total + kBlock - 1) / kBlock), kBlock, 0, stream>>>(
-        *grid, *a, S.F, S.mask[0], S.mask[1], S.L, S.faces, DcFuse{});
+        *grid, *a, S.F, S.mask[0], S.mask[1], S.L, S.faces);
     return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
 }
 
-// carve + the assembly that also writes the mixed-precision form's first
-// cycle (records, r', x^2 partials); *nparts: the number of partials
-template <class Args, class FacesK, class AssembleK>
-static int setup_transport_dc(const TseGrid* grid, const Args* a, void* d_ws, size_t ws_bytes,
-                              cudaStream_t stream, FacesK fk, AssembleK kernel, int imbl,
-                              TransportSetup& S, int* nparts) {
-    int rc = carve_transport(grid, a, d_ws, ws_bytes, stream, imbl, S);
-    if (rc != TSE_OK) return rc;
-    if (S.tail_bytes < dc_extra_bytes(S.L)) return TSE_ERR_WORKSPACE;
-    launch_faces(grid, a, S, fk, stream);
+// the mixed-precision form's assembly of a carved setup, for the given dt
+template <class Kind>
+static int assemble_fast(const TseGrid* grid, const typename Kind::Args* a, TransportSetup& S, int* nparts,
+                         cudaStream_t stream) {
     DcCtl c;
     dc_carve(S, c, TA_X);
     long long per, nb;
@@ -600,34 +816,66 @@ static int setup_transport_dc(const TseGrid* grid, const Args* a, void* d_ws, si
     fz.ks = c.ks;
     fz.partials = S.partials;
     fz.per_thread = (int)per;
-    kernel<<<(unsigned)nb, kBlock, 0, stream>>>(*grid, *a, S.F, S.mask[0], S.mask[1], S.L, S.faces,
-                                                 fz);
+    double2* tab = (double2*)S.faces;
+    const int nt = S.L.nx + S.L.ny + S.L.nz;
+    axis_tables_kernel<<<(unsigned)((nt + 127) / 128), 128, 0, stream>>>(*grid, tab);
+    // the form as the assembly fills it: with `lean` its later sums read one
+    // fixed term (setup_transport_dc), its own switches say what goes in
+    TransportForm F = S.F;
+    F.useY = a->omega != 1.0;
+    F.useEX = a->imblflo != 0;
+    if (S.lean)
+        assemble_fast_kernel<Kind, true><<<(unsigned)nb, kBlock, 0, stream>>>(*grid, *a, F, S.mask[0], S.mask[1],
+                                                                               S.L, tab, fz);
+    else
+        assemble_fast_kernel<Kind, false><<<(unsigned)nb, kBlock, 0, stream>>>(*grid, *a, F, S.mask[0],
+                                                                                S.mask[1], S.L, tab, fz);
     *nparts = (int)nb;
     return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
+}
+
+// carve + the mixed-precision form's assembly; *nparts: the number of x^2
+// partials.  S.lean: see SolveSetup.
+template <class Kind>
+static int setup_transport_dc(const TseGrid* grid, const typename Kind::Args* a, void* d_ws, size_t ws_bytes,
+                              cudaStream_t stream, TransportSetup& S, int* nparts) {
+    int rc = carve_transport(grid, a, d_ws, ws_bytes, stream, a->imblflo, S);
+    if (rc != TSE_OK) return rc;
+    if (S.tail_bytes < dc_extra_bytes(S.L)) return TSE_ERR_WORKSPACE;
+    if (S.lean) S.F.useY = S.F.useEX = S.F.useW = 0;
+    return assemble_fast<Kind>(grid, a, S, nparts, stream);
 }
 
 int setup_species(const TseGrid* grid, const TseSpeciesArgs* a, void* d_ws, size_t ws_bytes,
                   cudaStream_t stream, TransportSetup& S) {
     return setup_transport(grid, a, d_ws, ws_bytes, stream, faces_kernel<SpeciesKind>,
-                           assemble_c_kernel<false>, a->imblflo, S);
+                           assemble_c_kernel, a->imblflo, S);
 }
 
 int setup_heat(const TseGrid* grid, const TseHeatArgs* a, void* d_ws, size_t ws_bytes,
                cudaStream_t stream, TransportSetup& S) {
     return setup_transport(grid, a, d_ws, ws_bytes, stream, faces_kernel<HeatKind>,
-                           assemble_t_kernel<false>, a->imblflo, S);
+                           assemble_t_kernel, a->imblflo, S);
 }
 
 int setup_species_dc(const TseGrid* grid, const TseSpeciesArgs* a, void* d_ws, size_t ws_bytes,
                      cudaStream_t stream, TransportSetup& S, int* nparts) {
-    return setup_transport_dc(grid, a, d_ws, ws_bytes, stream, faces_kernel<SpeciesKind>,
-                              assemble_c_kernel<true>, a->imblflo, S, nparts);
+    return setup_transport_dc<SpeciesFast>(grid, a, d_ws, ws_bytes, stream, S, nparts);
 }
 
 int setup_heat_dc(const TseGrid* grid, const TseHeatArgs* a, void* d_ws, size_t ws_bytes,
                   cudaStream_t stream, TransportSetup& S, int* nparts) {
-    return setup_transport_dc(grid, a, d_ws, ws_bytes, stream, faces_kernel<HeatKind>,
-                              assemble_t_kernel<true>, a->imblflo, S, nparts);
+    return setup_transport_dc<HeatFast>(grid, a, d_ws, ws_bytes, stream, S, nparts);
+}
+
+int again_species_dc(const TseGrid* grid, const TseSpeciesArgs* a, cudaStream_t stream, TransportSetup& S,
+                     int* nparts) {
+    return assemble_fast<SpeciesFast>(grid, a, S, nparts, stream);
+}
+
+int again_heat_dc(const TseGrid* grid, const TseHeatArgs* a, cudaStream_t stream, TransportSetup& S,
+                  int* nparts) {
+    return assemble_fast<HeatFast>(grid, a, S, nparts, stream);
 }
 
 template <class Args, class FacesK, class AssembleK>
@@ -733,7 +981,7 @@ extern "C" int32_t tse_compute_C(const TseGrid* grid, const TseSpeciesArgs* a,
         !a->qz || !a->BC || !a->WC || !a->RC || !a->e || !a->l_l || !a->l_t)
         return TSE_ERR_ARG;
     return run_transport(grid, a, a->C, d_status, d_ws, ws_bytes, stream, faces_kernel<SpeciesKind>,
-                         assemble_c_kernel<false>, a->imblflo);
+                         assemble_c_kernel, a->imblflo);
 }
 
 extern "C" int32_t tse_compute_T(const TseGrid* grid, const TseHeatArgs* a,
@@ -745,7 +993,7 @@ extern "C" int32_t tse_compute_T(const TseGrid* grid, const TseHeatArgs* a,
         !a->BT || !a->WT || !a->e || !a->l_r || !a->rho_r || !a->cp_r || !a->l_l || !a->l_t)
         return TSE_ERR_ARG;
     return run_transport(grid, a, a->T, d_status, d_ws, ws_bytes, stream, faces_kernel<HeatKind>,
-                         assemble_t_kernel<false>, a->imblflo);
+                         assemble_t_kernel, a->imblflo);
 }
 
 extern "C" int32_t tse_smolarkiewicz(const TseGrid* grid, const double* C, const double* qx,
