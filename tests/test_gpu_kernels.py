@@ -7,6 +7,7 @@ kernels keep the reference's operation order, so most fields agree bit for
 bit; only the L2 sums are reduced in a different order (tree vs sequential)."""
 import numpy
 import pytest
+import torch
 
 from oracle.oracle import OracleModel
 from tests.golden import cases
@@ -227,3 +228,74 @@ def test_declared_eos_forms_bit_exact(cuda_device):
         for c in numpy.ndindex(shp):
             want[c] = eos.eval_form_host(d, [0.0, 0.0, guard[c]], T[c], old[c])
         assert numpy.array_equal(got, want), d
+
+
+def _same_bits(a, b):
+    real = ~numpy.isnan(b)
+    return (numpy.array_equal(a, b, equal_nan=True)
+            and numpy.array_equal(numpy.signbit(a)[real], numpy.signbit(b)[real]))
+
+
+# a thread a cell; then walks along x: planes of fewer cells than a warp's, of a warp's outputs
+# (30, 31) and one more, of several blocks, walks of one cell, with a remainder, the longest
+FLOW_SHAPES = [(1, 1, 1), (1, 1, 40), (40, 1, 3), (33, 17, 62), (61, 80, 83), (410000, 1, 3), (42000, 5, 6),
+               (40000, 31, 1), (38000, 4, 8), (250, 40, 125), (3, 500, 803)]
+
+
+@pytest.mark.parametrize("extremes", [False, True])
+@pytest.mark.parametrize("shape", FLOW_SHAPES)
+def test_flow_passes_match_the_oracle_bit_for_bit(shape, extremes, cuda_device):
+    """Fluxes, flow error and CFL step: divisors shared through reciprocals
+    give the divided quotients; zeros, infinities, NaN and magnitudes near the
+    ends of the exponent range included."""
+    cfg, rng = _random_case(shape, sum(shape))
+
+    def spread(x):
+        x = numpy.ascontiguousarray(x)
+        if extremes:
+            for v in (0.0, -0.0, 1e-310, 3e-200, 7e250, numpy.inf, numpy.nan, 1.0):
+                x[rng.uniform(size=shape) < 0.004] = v
+        return x
+
+    K = [spread(1e-12 * numpy.exp(2 * rng.standard_normal(shape))) for _ in range(3)]
+    nue, rho = spread(rng.uniform(8e-4, 1.2e-3, shape)), spread(rng.uniform(995, 1150, shape))
+    phi, c_f = spread(rng.uniform(0.05, 0.3, shape)), spread(4.5e-10 * rng.uniform(0.5, 1.5, shape))
+    P = spread(1e5 + 300 * rng.standard_normal(shape))
+    P[rng.uniform(size=shape) < 0.1] = 1e5
+    Pn = P + rng.standard_normal(shape)
+    BP = (rng.uniform(size=shape) < 0.4).astype(float)
+    WP = numpy.where(rng.uniform(size=shape) < 0.2, rng.uniform(-1e-4, 1e-4, shape), 0.0)
+    q0 = [spread(rng.uniform(-1e-5, 1e-5, shape) * 10.0 ** rng.integers(-12, 6, shape)) for _ in range(3)]
+    orc, m = OracleModel(cfg), model_for(cfg, cuda_device)
+    nk = NumpyKernels(m)
+    with numpy.errstate(all="ignore"):
+        qo = orc.compute_q(P, BP, *K, *[x.copy() for x in q0], nue, rho)
+        eo = orc.flow_error(P, Pn, *q0, WP, phi, c_f, cfg.c_r, rho, 3600.0)
+        to = orc.dt_cfl(*q0, phi)
+    qg = nk.compute_q(P, BP, *K, *[x.copy() for x in q0], nue, rho)
+    for a, b in zip(qg, qo):
+        assert _same_bits(a, b)
+    assert _same_bits(nk.flow_error(P, Pn, *q0, WP, phi, c_f, cfg.c_r, rho, 3600.0), eo)
+    assert numpy.array_equal(m.dt_cfl(*q0, phi), to, equal_nan=True)
+    fin = [numpy.where(numpy.isfinite(x), x, 0.0) for x in (*q0, phi)]
+    with numpy.errstate(all="ignore"):
+        assert numpy.array_equal(m.dt_cfl(*fin), orc.dt_cfl(*fin), equal_nan=True)
+
+
+@pytest.mark.parametrize("ns", range(9))
+def test_mass_totals_for_every_species_count(ns, cuda_device):
+    shape = (37, 41, 29)
+    cfg, rng = _random_case(shape, ns)
+    f = [rng.uniform(0.1, 2, shape) for _ in range(9)]
+    C, WC = ([rng.uniform(0, 1, shape) for _ in range(ns)] for _ in range(2))
+    phi, rho, RC, T, cp_f, rho_r, cp_r, WP, WT = f
+    V = cfg.dx[:, None, None] * cfg.dy[None, :, None] * cfg.dz[None, None, :]
+    want = [phi * rho, *[RC * phi * c for c in C], (phi * rho * cp_f + (1 - phi) * rho_r * cp_r) * T, WP, *WC, WT]
+    m = model_for(cfg, cuda_device)
+    dev = [m._t(torch.as_tensor(x, device=cuda_device)) for x in f + C + WC]
+    got = m.mass_totals(*dev[:3], dev[9:9 + ns], dev[9 + ns:], *dev[3:9])
+    assert len(got) == 2 * ns + 4
+    # sums of n positive terms, each side's rounding below n / 2 units of 2^-52
+    for a, b in zip(got, want):
+        b = (b * V).sum()
+        assert abs(a - b) <= 1e-12 * b

@@ -1,6 +1,9 @@
 // Darcy fluxes, flow-balance error, CFL / Neumann limits, L2 norm, field
 // statistics, Peclet diagnostics and the declared linear EOS.
 // FP64, reference operation order, compiled with --fmad=false.
+#include <algorithm>
+#include <cmath>
+
 #include "tse_common.cuh"
 
 namespace tse {
@@ -12,15 +15,114 @@ __device__ __forceinline__ void decode(long long t, int ny, int nz, int& i, int&
     grid_coords(t, ny, nz, i, j, k, row);
 }
 
+// ------------------------------------------------------ exact quotients
+// FP64 divisions bound the two flux kernels, 26 a cell in compute_q and 25 in
+// flow_error by the formulas: an operator's branch for special operands keeps
+// one from overlapping the next, and each does its own reciprocal.  Here a
+// reciprocal is formed once a divisor and correctly rounded, and quotients by
+// it take two fused corrections (Markstein 1990, "Computation of elementary
+// functions on the IBM RISC System/6000": from a faithful y,
+// y + (1 - b y) y = RN(1 / b) unless b's significand is all ones, and from a
+// faithful q and that y, q + (a - b q) y = RN(a / b)), without a branch.  The
+// results are the divided quotients' bits as long as no operand is near an end
+// of the exponent range; a cell that has another operand is formed by the
+// formulas' own divisions (*_cell).
+struct Divisor {
+    double b, y;
+};
+__device__ __forceinline__ Divisor divisor(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));   // to 2^-20
+    const double e = __fma_rn(-b, y, 1.0);
+    y = __fma_rn(y, __fma_rn(e, e, e), y);
+    return {b, __fma_rn(__fma_rn(-b, y, 1.0), y, y)};
+}
+__device__ __forceinline__ double quotient(double a, const Divisor& d) {
+    double q = a * d.y;
+    q = __fma_rn(__fma_rn(-d.b, q, a), d.y, q);
+    return __fma_rn(__fma_rn(-d.b, q, a), d.y, q);
+}
+// a may be zero: keeps its sign
+__device__ __forceinline__ double quotient_0(double a, const Divisor& d) {
+    return a == 0.0 ? a * d.y : quotient(a, d);
+}
+__device__ __forceinline__ Divisor half(const Divisor& s) { return {0.5 * s.b, 2.0 * s.y}; }
+// positive, within 2^-80 .. 2^80: what the formulas derive from such inputs
+// stays within 2^-900 .. 2^900
+__device__ __forceinline__ bool plain_positive(double v) {
+    return (unsigned)__double2hiint(v) - (943u << 20) <= (160u << 20);
+}
+// 0 or of magnitude 2^-300 .. 2^300
+__device__ __forceinline__ bool plain_signed(double v) {
+    return v == 0.0 || ((unsigned)__double2hiint(v) & 0x7fffffffu) - (723u << 20) <= (600u << 20);
+}
+__device__ __forceinline__ bool not_all_ones(double b) { return __double2loint(b) != -1; }
+__device__ __forceinline__ bool plain_divisor(double b) { return plain_positive(b) && not_all_ones(b); }
+
+// The flux kernels walk along x with a warp on 32 consecutive cells of the
+// (y, z) plane: the x face and its quotients stay in registers, a z face's come
+// from the next lane (rows need no alignment: a row's last cell has no + face),
+// and reciprocals of spacings are formed once a walk.  Lanes at a warp's ends
+// repeat cells of the next one.
+constexpr int kWalkMax = 16;
+// From these grid sizes on; below, a thread a cell keeps the SMs fuller (us,
+// thread a cell against walks: fluxes 31 / 33 at 96^3, 56 / 51 at 112^3, 130 / 105
+// at 160 x 192 x 101; flow error 5.2 / 6.5 at 48^3, 16 / 14 at 80^3, 99 / 75).
+constexpr long long kWalkCellsQ = 1200000, kWalkCellsE = 400000;
+constexpr int kWalkBlocksQ = 4, kWalkBlocksE = 3;   // resident on a SM
+constexpr int kWalkWarps = kBlock / 32;
+struct Walk {
+    int steps;                // cells of a walk
+    unsigned tiles, blocks;   // blocks across the plane, and of all walks
+};
+// The length whose waves of resident blocks take the fewest steps in all, one
+// more a walk for its start (a last wave that is nearly empty costs a full one).
+static Walk walk_of(const TseGrid& g, int out_lanes, int blocks_per_sm) {
+    const long long plane = (long long)g.ny * g.nz;
+    const long long warps = (plane + out_lanes - 1) / out_lanes, slots = 148LL * blocks_per_sm;
+    Walk w = {1, (unsigned)((warps + kWalkWarps - 1) / kWalkWarps), 0};
+    long long best = 0;
+    for (int s = kWalkMax; s >= 1; --s) {
+        const long long blocks = (long long)w.tiles * ((g.nx + s - 1) / s);
+        const long long cost = (blocks + slots - 1) / slots * (s + 1);
+        if (best == 0 || cost < best) {
+            best = cost;
+            w.steps = s;
+            w.blocks = (unsigned)blocks;
+        }
+    }
+    return w;
+}
+// along x: spacings dx[i0 - 1 .. i0 + steps] and the divisors dx[i] and
+// dx[i] + dx[i + 1] of cells i0 - 1 .. (spacing 1 beside the grid, unused)
+struct WalkX {
+    double d[kWalkMax + 2];
+    Divisor own[kWalkMax + 1], sum[kWalkMax + 1];
+    // false in every thread if a divisor is not plain
+    __device__ __forceinline__ bool fill(const TseGrid& g, int i0) {
+        bool ok = true;
+        for (int q = threadIdx.x; q < kWalkMax + 2; q += blockDim.x) {
+            const int i = i0 - 1 + q;
+            const double a = i >= 0 && i < g.nx ? g.dx[i] : 1.0;
+            d[q] = a;
+            ok = ok && plain_divisor(a);
+            if (q < kWalkMax + 1) {
+                const double b = i + 1 < g.nx ? g.dx[i + 1] : 1.0;
+                own[q] = divisor(a);
+                sum[q] = divisor(b + a);
+                ok = ok && plain_divisor(b + a);
+            }
+        }
+        return __syncthreads_and(ok);
+    }
+};
+
 // compute_q (tse.py:744-780); q on the last plane of each axis is not written
-__global__ void compute_q_kernel(TseGrid g, const double* P, const double* BP, const double* Kx,
-                                 const double* Ky, const double* Kz, double* qx, double* qy,
-                                 double* qz, const double* nue, const double* rho) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void darcy_cell(const TseGrid& g, long long t, int i, int j, int k, const double* P,
+                                           const double* BP, const double* Kx, const double* Ky,
+                                           const double* Kz, double* qx, double* qy, double* qz,
+                                           const double* nue, const double* rho) {
     const int nx = g.nx, ny = g.ny, nz = g.nz;
-    if (t >= (long long)nx * ny * nz) return;
-    int i, j, k;
-    decode(t, ny, nz, i, j, k);
     const double *dx = g.dx, *dy = g.dy, *dz = g.dz;
     if (i < nx - 1) {
         const long long o = t + (long long)ny * nz;
@@ -50,16 +152,127 @@ __global__ void compute_q_kernel(TseGrid g, const double* P, const double* BP, c
     }
 }
 
-// flow_error (tse.py:409-446)
-__global__ void flow_error_kernel(TseGrid g, const double* P, const double* Pn, const double* qx,
-                                  const double* qy, const double* qz, const double* WP,
-                                  const double* phi, const double* c_f, const double* c_r,
-                                  const double* rho, double dt_P, double* e) {
+__device__ __noinline__ void compute_q_cell(const TseGrid& g, long long t, int i, int j, int k, const double* P,
+                                            const double* BP, const double* Kx, const double* Ky,
+                                            const double* Kz, double* qx, double* qy, double* qz,
+                                            const double* nue, const double* rho) {
+    darcy_cell(g, t, i, j, k, P, BP, Kx, Ky, Kz, qx, qy, qz, nue, rho);
+}
+__global__ void compute_q_cells_kernel(TseGrid g, const double* P, const double* BP, const double* Kx,
+                                       const double* Ky, const double* Kz, double* qx, double* qy, double* qz,
+                                       const double* nue, const double* rho) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int nx = g.nx, ny = g.ny, nz = g.nz;
-    if (t >= (long long)nx * ny * nz) return;
+    if (t >= (long long)g.nx * g.ny * g.nz) return;
     int i, j, k;
-    decode(t, ny, nz, i, j, k);
+    decode(t, g.ny, g.nz, i, j, k);
+    darcy_cell(g, t, i, j, k, P, BP, Kx, Ky, Kz, qx, qy, qz, nue, rho);
+}
+
+// A K of zero (harm2 is then 0) goes along as 1 and a flag.
+struct Perm {
+    double a;   // d / K
+    bool zero;
+};
+__device__ __forceinline__ Perm perm(double K, double d, bool& ok) {
+    const bool z = K == 0.0;
+    const double s = z ? 1.0 : K;
+    ok = ok && plain_divisor(s);
+    return {quotient(d, divisor(s)), z};
+}
+// -harm2(K) / harm2(nue) of a face
+__device__ __forceinline__ double mobility(double dsum, const Perm& a, const Perm& b, double n1, double n2,
+                                           bool& ok) {
+    const double sk = a.a + b.a, sn = n1 + n2;
+    const double hk = quotient(dsum, divisor(sk)), hn = quotient(dsum, divisor(sn));
+    ok = ok && not_all_ones(sk) && not_all_ones(sn) && not_all_ones(hn);
+    return quotient_0(a.zero || b.zero ? -0.0 : -hk, divisor(hn));
+}
+
+// 255 x 256 x 127 (B200): 418 us with a thread a cell and the operator's
+// divisions, 265 now (10 arrays, 101 us); a tenth more with 2 or 3 blocks a SM or
+// with 5.  Bound: FP64 arithmetic, 15 reciprocals and 23 quotients a cell.
+__global__ void __launch_bounds__(kBlock, kWalkBlocksQ)
+    compute_q_kernel(TseGrid g, Walk w, const double* P, const double* BP, const double* Kx, const double* Ky,
+                     const double* Kz, double* qx, double* qy, double* qz, const double* nue,
+                     const double* rho) {
+    __shared__ WalkX X;
+    const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const long long plane = (long long)ny * nz;
+    const int i0 = (int)(blockIdx.x / w.tiles) * w.steps, tile = (int)(blockIdx.x % w.tiles);
+    bool okd = X.fill(g, i0);
+    const int lane = threadIdx.x & 31;
+    const long long u = ((long long)tile * kWalkWarps + (threadIdx.x >> 5)) * 31 + lane;
+    if (u - lane >= plane) return;   // whole warps only: the others exchange
+    const bool out = u < plane && lane < 31;
+    const long long c0 = u < plane ? u : plane - 1;
+    const int j = (int)(c0 / nz), k = (int)(c0 - (long long)j * nz);
+    const bool hy = j < ny - 1, hz = k < nz - 1;
+    const double dy0 = g.dy[j], dy1 = hy ? g.dy[j + 1] : 1.0, dz0 = g.dz[k], dz1 = hz ? g.dz[k + 1] : 1.0;
+    const Divisor sy = divisor(dy1 + dy0), sz = divisor(dz1 + dz0);
+    okd = okd && plain_positive(dy0) && plain_positive(dy1) && plain_positive(dz0) && plain_positive(dz1) &&
+          plain_divisor(sy.b) && plain_divisor(sz.b);
+    long long t = (long long)i0 * plane + c0;
+    double p = P[t], r = rho[t], n = nue[t], bp = BP[t];
+    bool ok0 = okd && plain_divisor(n) && plain_positive(r);   // the cell's own values
+    Divisor nd = divisor(n);
+    Perm ax = perm(Kx[t], X.d[1], ok0);
+    double an = quotient(X.d[1], nd);
+    const int steps = min(w.steps, nx - i0);
+    for (int s = 0; s < steps; ++s, t += plane) {
+        const bool hx = i0 + s < nx - 1;
+        const long long tx = hx ? t + plane : t, ty = hy ? t + nz : t, tz = hz ? t + 1 : t;
+        // the next cell along x, and this cell's + neighbours along y and z
+        const double p1 = P[tx], r1 = rho[tx], n1 = nue[tx], kx1 = Kx[tx], b1 = BP[tx];
+        const double ky = Ky[t], kz = Kz[t], kyo = Ky[ty], no = nue[ty], po = P[ty], bo = BP[ty];
+        const double pz = P[tz], rz = rho[tz], bz = BP[tz];
+        const Divisor nd1 = divisor(n1);
+        bool ok1 = okd && plain_divisor(n1) && plain_positive(r1);
+        const Perm ax1 = perm(kx1, X.d[s + 2], ok1);
+        const double an1 = quotient(X.d[s + 2], nd1);
+        bool ok = ok0 && ok1 && plain_divisor(no) && plain_positive(rz);
+        Perm zk = perm(kz, dz0, ok);
+        const double zn = quotient(dz0, nd);
+        const unsigned good = __ballot_sync(0xffffffffu, ok), zero = __ballot_sync(0xffffffffu, zk.zero);
+        const Perm zk1 = {__shfl_down_sync(0xffffffffu, zk.a, 1), (zero >> ((lane + 1) & 31) & 1u) != 0};
+        const double zn1 = __shfl_down_sync(0xffffffffu, zn, 1);
+        ok = ok && (!hz || (good >> ((lane + 1) & 31) & 1u));
+        const double px = p1 - p, py = po - p, pu = pz - p;
+        ok = ok && plain_signed(px) && plain_signed(py) && plain_signed(pu);
+        const Divisor sx = X.sum[s + 1];
+        const double vx = mobility(sx.b, ax1, ax, an1, an, ok) *
+                          (quotient_0(px, half(sx)) + quotient(r1 * X.d[s + 2] + r * X.d[s + 1], sx) * g.g * g.sin_beta);
+        const double vy = quotient_0(mobility(sy.b, perm(kyo, dy1, ok), perm(ky, dy0, ok), quotient(dy1, divisor(no)),
+                                              quotient(dy0, nd), ok) * py,
+                                     half(sy));
+        const double vz = mobility(sz.b, zk1, zk, zn1, zn, ok) *
+                          (quotient_0(pu, half(sz)) + quotient(rz * dz1 + r * dz0, sz) * g.g * g.cos_beta);
+        if (out) {
+            if (ok) {
+                const bool in = bp != 0;
+                if (hx) qx[t] = in && b1 != 0 ? 0.0 : vx;
+                if (hy) qy[t] = in && bo != 0 ? 0.0 : vy;
+                if (hz) qz[t] = in && bz != 0 ? 0.0 : vz;
+            } else {
+                compute_q_cell(g, t, i0 + s, j, k, P, BP, Kx, Ky, Kz, qx, qy, qz, nue, rho);
+            }
+        }
+        p = p1;
+        r = r1;
+        bp = b1;
+        nd = nd1;
+        ax = ax1;
+        an = an1;
+        ok0 = ok1;
+    }
+}
+
+// flow_error (tse.py:409-446)
+__device__ __forceinline__ double balance_cell(const TseGrid& g, long long t, int i, int j, int k, const double* P,
+                                               const double* Pn, const double* qx, const double* qy,
+                                               const double* qz, const double* WP, const double* phi,
+                                               const double* c_f, const double* c_r, const double* rho,
+                                               double dt_P) {
+    const int nx = g.nx, ny = g.ny, nz = g.nz;
     const double *dx = g.dx, *dy = g.dy, *dz = g.dz;
     const long long sx = (long long)ny * nz;
     double v = 0.0;
@@ -71,7 +284,113 @@ __global__ void flow_error_kernel(TseGrid g, const double* P, const double* Pn, 
     if (k != 0) v += (qz[t - 1] / dz[k] * harm2(rho[t - 1], rho[t], dz[k - 1], dz[k]));
     const double por = phi[t];
     v += (WP[t] + ((1 - por) * c_r[t] + por * c_f[t]) * (P[t] - Pn[t]) * rho[t] / dt_P);
-    e[t] = v;
+    return v;
+}
+
+__device__ __noinline__ double flow_error_cell(const TseGrid& g, long long t, int i, int j, int k, const double* P,
+                                               const double* Pn, const double* qx, const double* qy,
+                                               const double* qz, const double* WP, const double* phi,
+                                               const double* c_f, const double* c_r, const double* rho,
+                                               double dt_P) {
+    return balance_cell(g, t, i, j, k, P, Pn, qx, qy, qz, WP, phi, c_f, c_r, rho, dt_P);
+}
+__global__ void flow_error_cells_kernel(TseGrid g, const double* P, const double* Pn, const double* qx,
+                                        const double* qy, const double* qz, const double* WP, const double* phi,
+                                        const double* c_f, const double* c_r, const double* rho, double dt_P,
+                                        double* e) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)g.nx * g.ny * g.nz) return;
+    int i, j, k;
+    decode(t, g.ny, g.nz, i, j, k);
+    e[t] = balance_cell(g, t, i, j, k, P, Pn, qx, qy, qz, WP, phi, c_f, c_r, rho, dt_P);
+}
+
+// harm2 from its two quotients
+__device__ __forceinline__ double harm_of(double dsum, double a1, double a2, bool& ok) {
+    ok = ok && not_all_ones(a1 + a2);
+    return quotient(dsum, divisor(a1 + a2));
+}
+
+// A face's mean density is the same bits from either side.  255 x 256 x 127
+// (B200): 305 us before, 190 now (11 arrays, 112 us); a tenth more with 2 blocks a SM
+// or with 4.  Bound: FP64 arithmetic, 7 reciprocals and 18 quotients a cell.
+__global__ void __launch_bounds__(kBlock, kWalkBlocksE)
+    flow_error_kernel(TseGrid g, Walk w, const double* P, const double* Pn, const double* qx, const double* qy,
+                      const double* qz, const double* WP, const double* phi, const double* c_f,
+                      const double* c_r, const double* rho, double dt_P, double* e) {
+    __shared__ WalkX X;
+    const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const long long plane = (long long)ny * nz;
+    const int i0 = (int)(blockIdx.x / w.tiles) * w.steps, tile = (int)(blockIdx.x % w.tiles);
+    bool okd = X.fill(g, i0);
+    const int lane = threadIdx.x & 31;
+    const long long u = ((long long)tile * kWalkWarps + (threadIdx.x >> 5)) * 30 + lane - 1;
+    if (u - lane + 1 >= plane) return;   // whole warps only: the others exchange
+    const bool out = u >= 0 && u < plane && lane > 0 && lane < 31;
+    const long long c0 = u < 0 ? 0 : u < plane ? u : plane - 1;
+    const int j = (int)(c0 / nz), k = (int)(c0 - (long long)j * nz);
+    const bool hy = j < ny - 1, ly = j != 0, hz = k < nz - 1, lz = k != 0;
+    const double dy1 = hy ? g.dy[j + 1] : 1.0, dy2 = ly ? g.dy[j - 1] : 1.0;
+    const double dz1 = hz ? g.dz[k + 1] : 1.0;
+    const Divisor dy = divisor(g.dy[j]), dz = divisor(g.dz[k]), dt = divisor(dt_P);
+    okd = okd && plain_divisor(dy.b) && plain_divisor(dz.b) && plain_divisor(dt_P) && plain_positive(dy1) &&
+          plain_positive(dy2) && plain_positive(dz1);
+    long long t = (long long)i0 * plane + c0;
+    double r = rho[t];
+    bool ok0 = okd && plain_divisor(r), okm = true;   // this cell's density; the face before
+    Divisor rd = divisor(r);
+    double ar = quotient(X.d[1], rd), q0 = 0.0, fx = 0.0;
+    if (i0 != 0) {
+        const double rm = rho[t - plane];
+        q0 = qx[t - plane];
+        okm = ok0 && plain_divisor(rm) && plain_signed(q0);
+        fx = harm_of(X.d[0] + X.d[1], quotient(X.d[0], divisor(rm)), ar, okm);
+    }
+    const int steps = min(w.steps, nx - i0);
+    for (int s = 0; s < steps; ++s, t += plane) {
+        const bool hx = i0 + s < nx - 1, lx = i0 + s != 0;
+        const double r1 = rho[hx ? t + plane : t], ra = rho[hy ? t + nz : t], rb = rho[ly ? t - nz : t];
+        const double fm = fx, qm = q0, qa = qy[t], qb = qy[ly ? t - nz : t], qu = qz[t], qd = qz[lz ? t - 1 : t];
+        q0 = qx[t];
+        const double por = phi[t], cr = c_r[t], cf = c_f[t], dp = P[t] - Pn[t], W = WP[t];
+        // the z face above, of this lane and of the one before
+        const double zr = quotient(dz.b, rd);
+        bool ok = ok0;
+        const double zr1 = __shfl_down_sync(0xffffffffu, zr, 1);
+        const double fz = harm_of(dz1 + dz.b, zr1, zr, ok);
+        const double fz0 = __shfl_up_sync(0xffffffffu, fz, 1);
+        // the lanes beside: their densities (and the face of the one before)
+        const unsigned good = __ballot_sync(0xffffffffu, ok);
+        ok = ok && (!hz || (good >> ((lane + 1) & 31) & 1u)) && (!lz || (good >> ((lane + 31) & 31) & 1u));
+        // the next x face
+        const Divisor rd1 = divisor(r1);
+        const bool ok1 = okd && plain_divisor(r1);
+        const double ar1 = quotient(X.d[s + 2], rd1);
+        bool okx = ok0 && ok1 && plain_signed(q0);
+        fx = harm_of(X.sum[s + 1].b, ar1, ar, okx);
+        ok = ok && okx && okm && plain_divisor(ra) && plain_divisor(rb) && plain_signed(qa) && plain_signed(qb) &&
+             plain_signed(qu) && plain_signed(qd);
+        const Divisor dx = X.own[s + 1];
+        const double yr = quotient(dy.b, rd);
+        const double fa = harm_of(dy1 + dy.b, quotient(dy1, divisor(ra)), yr, ok);
+        const double fb = harm_of(dy2 + dy.b, quotient(dy2, divisor(rb)), yr, ok);
+        double v = 0.0;
+        if (hx) v -= (quotient_0(q0, dx) * fx);
+        if (lx) v += (quotient_0(qm, dx) * fm);
+        if (hy) v -= (quotient_0(qa, dy) * fa);
+        if (ly) v += (quotient_0(qb, dy) * fb);
+        if (hz) v -= (quotient_0(qu, dz) * fz);
+        if (lz) v += (quotient_0(qd, dz) * fz0);
+        const double st = ((1 - por) * cr + por * cf) * dp * r;
+        ok = ok && plain_signed(st);
+        v += (W + quotient_0(st, dt));
+        if (out) e[t] = ok ? v : flow_error_cell(g, t, i0 + s, j, k, P, Pn, qx, qy, qz, WP, phi, c_f, c_r, rho, dt_P);
+        okm = okx;
+        r = r1;
+        rd = rd1;
+        ar = ar1;
+        ok0 = ok1;
+    }
 }
 
 // ---------------------------------------------------------------- reduces
@@ -100,11 +419,19 @@ struct Ops {
 __global__ void finish_kernel(const double* parts, int nparts, int nout, Ops ops, double* out,
                               int post) {
     __shared__ double sh[kBlock / 32];
-    for (int q = 0; q < nout; ++q) {
-        const int op = ops.op[q];
-        double v = red_init(op);
-        for (int b = threadIdx.x; b < nparts; b += blockDim.x) v = red_combine(op, v, parts[q * nparts + b]);
-        double r = block_red<kBlock>(op, v, sh);
+    // every output's loads before the first reduction
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        v[q] = red_init(ops.op[q]);
+        if (q < nout)
+#pragma unroll 4
+            for (int b = threadIdx.x; b < nparts; b += kBlock) v[q] = red_combine(ops.op[q], v[q], parts[q * nparts + b]);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (q >= nout) break;
+        double r = block_red<kBlock>(ops.op[q], v[q], sh);
         if (threadIdx.x == 0) out[q] = r;
         __syncthreads();
     }
@@ -137,22 +464,51 @@ __global__ void l2_partial_kernel(const double* New, const double* Old, long lon
 
 // dt_CFL (tse.py:1241-1246): element f of reshape(|qx|/phi, (ny,nz,nx)) / dx
 // is divided by dx[f % nx]; likewise dy[f % ny]; qz uses dz[k].
+// Bound: DRAM.  |q| / p / d is formed only where it can exceed the warp's
+// maximum so far (a product tells, with a margin for its rounding; anything
+// near an end of the exponent range, and NaN, is formed): of 160 us at
+// 255 x 256 x 127 the arrays take 41; six divisions and two 64-bit remainders a
+// cell took the rest.  Now 86.
+struct CflMax {
+    double m = -HUGE_VAL;   // the warp's
+    __device__ __forceinline__ bool below(double q, double p, double d) const {
+        const double mp = m * p, t = mp * d;
+        return mp < 1e290 && t > 1e-290 && t < 1e290 && q * (1.0 + 1e-12) < t;
+    }
+    __device__ __forceinline__ void take(double q, double p, double d, bool in) {
+        const bool cand = in && !below(q, p, d);
+        if (!__any_sync(0xffffffffu, cand)) return;
+        double v = cand ? q / p / d : m;
+        for (int o = 16; o > 0; o >>= 1) v = nmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+        m = nmax(m, v);
+    }
+};
 __global__ void cfl_partial_kernel(TseGrid g, const double* qx, const double* qy, const double* qz,
                                    const double* phi, double* parts) {
     __shared__ double sh[kBlock / 32];
     const long long n = (long long)g.nx * g.ny * g.nz;
-    const double ninf = -__longlong_as_double(0x7ff0000000000000LL);
-    double a = ninf, b = ninf, c = ninf;
-    for (long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x; f < n;
-         f += (long long)gridDim.x * blockDim.x) {
-        const double p = phi[f];
-        a = nmax(a, fabs(qx[f]) / p / g.dx[f % g.nx]);
-        b = nmax(b, fabs(qy[f]) / p / g.dy[f % g.ny]);
-        c = nmax(c, fabs(qz[f]) / p / g.dz[f % g.nz]);
+    const long long st = (long long)gridDim.x * blockDim.x, f0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    // f % nx, f % ny, f % nz, stepped along
+    const int ax = (int)(st % g.nx), ay = (int)(st % g.ny), az = (int)(st % g.nz);
+    int ix = (int)(f0 % g.nx), iy = (int)(f0 % g.ny), iz = (int)(f0 % g.nz);
+    CflMax a, b, c;
+    for (long long w0 = f0 - (threadIdx.x & 31), f = f0; w0 < n; w0 += st, f += st) {
+        const bool in = f < n;
+        const long long h = in ? f : n - 1;
+        const double p = phi[h], x = fabs(qx[h]), y = fabs(qy[h]), z = fabs(qz[h]);
+        a.take(x, p, g.dx[ix], in);
+        b.take(y, p, g.dy[iy], in);
+        c.take(z, p, g.dz[iz], in);
+        ix += ax;
+        iy += ay;
+        iz += az;
+        if (ix >= g.nx) ix -= g.nx;
+        if (iy >= g.ny) iy -= g.ny;
+        if (iz >= g.nz) iz -= g.nz;
     }
-    double ra = block_nmax<kBlock>(a, sh);
-    double rb = block_nmax<kBlock>(b, sh);
-    double rc = block_nmax<kBlock>(c, sh);
+    double ra = block_nmax<kBlock>(a.m, sh);
+    double rb = block_nmax<kBlock>(b.m, sh);
+    double rc = block_nmax<kBlock>(c.m, sh);
     if (threadIdx.x == 0) {
         parts[blockIdx.x] = ra;
         parts[gridDim.x + blockIdx.x] = rb;
@@ -280,45 +636,56 @@ struct MassArgs {
     const double *phi, *rho, *RC, *T, *cp_f, *rho_r, *cp_r, *WP, *WT;
     const double* C[8];
     const double* WC[8];
-    int ns;
 };
 
-__global__ void mass_partial_kernel(TseGrid g, MassArgs a, double* parts) {
+// Bound: DRAM.  One instance a species count, so the sums are registers: with
+// a run-time count they were local memory, 431 us at 255 x 256 x 127 and two
+// species, 141 now (13 arrays, 132 us).
+template <int NS>
+__global__ void __launch_bounds__(kBlock, 2) mass_partial_kernel(TseGrid g, MassArgs a, double* parts) {
     __shared__ double sh[kBlock / 32];
     const long long n = (long long)g.nx * g.ny * g.nz;
-    const int nq = 2 * a.ns + 4;
-    double acc[20];
-    for (int q = 0; q < 20; ++q) acc[q] = 0.0;
+    constexpr int nq = 2 * NS + 4;
+    double acc[nq];
+#pragma unroll
+    for (int q = 0; q < nq; ++q) acc[q] = 0.0;
     for (long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x; f < n;
          f += (long long)gridDim.x * blockDim.x) {
         int i, j, k;
         decode(f, g.ny, g.nz, i, j, k);
-        const double V = g.dx[i] * g.dy[j] * g.dz[k];
-        const double ph = a.phi[f];
-        acc[0] += ph * a.rho[f] * V;
-        for (int s = 0; s < a.ns; ++s) {
-            acc[1 + s] += a.RC[f] * ph * a.C[s][f] * V;
-            acc[a.ns + 3 + s] += a.WC[s][f] * V;
+        const double ph = a.phi[f], rho = a.rho[f], RC = a.RC[f], cf = a.cp_f[f], rr = a.rho_r[f], cr = a.cp_r[f],
+                     T = a.T[f], WP = a.WP[f], WT = a.WT[f];
+        double C[NS + 1], WC[NS + 1];
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            C[s] = a.C[s][f];
+            WC[s] = a.WC[s][f];
         }
-        acc[a.ns + 1] += (ph * a.rho[f] * a.cp_f[f] + (1 - ph) * a.rho_r[f] * a.cp_r[f]) * a.T[f] * V;
-        acc[a.ns + 2] += a.WP[f] * V;
-        acc[2 * a.ns + 3] += a.WT[f] * V;
+        const double V = g.dx[i] * g.dy[j] * g.dz[k];
+        acc[0] += ph * rho * V;
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            acc[1 + s] += RC * ph * C[s] * V;
+            acc[NS + 3 + s] += WC[s] * V;
+        }
+        acc[NS + 1] += (ph * rho * cf + (1 - ph) * rr * cr) * T * V;
+        acc[NS + 2] += WP * V;
+        acc[2 * NS + 3] += WT * V;
     }
+#pragma unroll
     for (int q = 0; q < nq; ++q) {
         const double r = block_sum<kBlock>(acc[q], sh);
         if (threadIdx.x == 0) parts[q * gridDim.x + blockIdx.x] = r;
     }
 }
 
-__global__ void mass_finish_kernel(const double* parts, int nparts, int nq, double* out) {
+// one block an output
+__global__ void mass_finish_kernel(const double* parts, int nparts, double* out) {
     __shared__ double sh[kBlock / 32];
-    for (int q = 0; q < nq; ++q) {
-        double v = 0.0;
-        for (int b = threadIdx.x; b < nparts; b += blockDim.x) v = v + parts[q * nparts + b];
-        const double r = block_sum<kBlock>(v, sh);
-        if (threadIdx.x == 0) out[q] = r;
-        __syncthreads();
-    }
+    double v = 0.0;
+    for (int b = threadIdx.x; b < nparts; b += kBlock) v = v + parts[(size_t)blockIdx.x * nparts + b];
+    const double r = block_sum<kBlock>(v, sh);
+    if (threadIdx.x == 0) out[blockIdx.x] = r;
 }
 
 // Declared linear EOS: rho = rho0 + a0*C[s0] + ... - tcoef*(T - T0)
@@ -404,8 +771,14 @@ extern "C" int32_t tse_compute_q(const TseGrid* grid, const double* P, const dou
     if (!grid || !P || !BP || !Kx || !Ky || !Kz || !qx || !qy || !qz || !nue || !rho_f) return TSE_ERR_ARG;
     const long long n = (long long)grid->nx * grid->ny * grid->nz;
     if (n <= 0) return TSE_ERR_ARG;
-    compute_q_kernel<<<grid_for(n), kBlock, 0, (cudaStream_t)stream>>>(*grid, P, BP, Kx, Ky, Kz, qx,
-                                                                       qy, qz, nue, rho_f);
+    if (n < kWalkCellsQ) {
+        compute_q_cells_kernel<<<grid_for(n), kBlock, 0, (cudaStream_t)stream>>>(*grid, P, BP, Kx, Ky, Kz, qx,
+                                                                                 qy, qz, nue, rho_f);
+        return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
+    }
+    const Walk w = walk_of(*grid, 31, kWalkBlocksQ);
+    compute_q_kernel<<<w.blocks, kBlock, 0, (cudaStream_t)stream>>>(*grid, w, P, BP, Kx, Ky, Kz, qx, qy, qz,
+                                                                  nue, rho_f);
     return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
 }
 
@@ -418,8 +791,14 @@ extern "C" int32_t tse_flow_error(const TseGrid* grid, const double* P, const do
         return TSE_ERR_ARG;
     const long long n = (long long)grid->nx * grid->ny * grid->nz;
     if (n <= 0) return TSE_ERR_ARG;
-    flow_error_kernel<<<grid_for(n), kBlock, 0, (cudaStream_t)stream>>>(*grid, P, Pn, qx, qy, qz, WP,
-                                                                        phi, c_f, c_r, rho_f, dt_P, e);
+    if (n < kWalkCellsE) {
+        flow_error_cells_kernel<<<grid_for(n), kBlock, 0, (cudaStream_t)stream>>>(
+            *grid, P, Pn, qx, qy, qz, WP, phi, c_f, c_r, rho_f, dt_P, e);
+        return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
+    }
+    const Walk w = walk_of(*grid, 30, kWalkBlocksE);
+    flow_error_kernel<<<w.blocks, kBlock, 0, (cudaStream_t)stream>>>(*grid, w, P, Pn, qx, qy, qz, WP, phi,
+                                                                   c_f, c_r, rho_f, dt_P, e);
     return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
 }
 
@@ -536,8 +915,8 @@ extern "C" int32_t tse_mass_totals(const TseGrid* grid, const double* phi, const
         return TSE_ERR_ARG;
     const long long n = (long long)grid->nx * grid->ny * grid->nz;
     const int nq = 2 * nspec + 4;
-    const unsigned nb = red_blocks(n) > 256 ? 256 : red_blocks(n);
-    if (ws_bytes < reduce_ws_bytes() || (size_t)nq * nb > (size_t)8 * kRedBlocks) return TSE_ERR_WORKSPACE;
+    const unsigned nb = std::min(red_blocks(n), 256u);   // nq nb partials fit the workspace
+    if (ws_bytes < reduce_ws_bytes()) return TSE_ERR_WORKSPACE;
     MassArgs a;
     a.phi = phi;
     a.rho = rho_f;
@@ -548,16 +927,19 @@ extern "C" int32_t tse_mass_totals(const TseGrid* grid, const double* phi, const
     a.cp_r = cp_r;
     a.WP = WP;
     a.WT = WT;
-    a.ns = nspec;
     for (int s = 0; s < 8; ++s) {
         a.C[s] = s < nspec ? h_C[s] : nullptr;
         a.WC[s] = s < nspec ? h_WC[s] : nullptr;
     }
     cudaStream_t s = (cudaStream_t)stream;
     double* parts = (double*)ws;
-    mass_partial_kernel<<<nb, kBlock, 0, s>>>(*grid, a, parts);
+    using Kernel = void (*)(TseGrid, MassArgs, double*);
+    static const Kernel kernels[9] = {mass_partial_kernel<0>, mass_partial_kernel<1>, mass_partial_kernel<2>,
+                                      mass_partial_kernel<3>, mass_partial_kernel<4>, mass_partial_kernel<5>,
+                                      mass_partial_kernel<6>, mass_partial_kernel<7>, mass_partial_kernel<8>};
+    kernels[nspec]<<<nb, kBlock, 0, s>>>(*grid, a, parts);
     if (cudaGetLastError() != cudaSuccess) return TSE_ERR_LAUNCH;
-    mass_finish_kernel<<<1, kBlock, 0, s>>>(parts, (int)nb, nq, d_out);
+    mass_finish_kernel<<<nq, kBlock, 0, s>>>(parts, (int)nb, d_out);
     return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
 }
 

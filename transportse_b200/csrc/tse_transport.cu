@@ -936,10 +936,9 @@ __global__ void smolarkiewicz_kernel(TseGrid g, const double* C, const double* q
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     const long long total = (long long)nx * ny * nz;
     if (t >= total) return;
-    const int k = (int)(t % nz);
-    const long long row = t / nz;
-    const int j = (int)(row % ny);
-    const int i = (int)(row / ny);
+    int i, j, k;
+    long long row;
+    grid_coords(t, ny, nz, i, j, k, row);
     const double c0 = C[t];
     if (c0 > 0) {
         double dd;
