@@ -630,3 +630,21 @@ def test_face_means_are_the_same_from_either_cell():
     lr_s, lf_s = harm2(H2, H1, d2, d1), harm2(H1 * 7, H2 * 3, d2, d1)
     por_s = amean2(X2, X1, d2, d1) * 1e-4
     assert numpy.array_equal((1 - por) * lr + por * lf, (1 - por_s) * lr_s + por_s * lf_s)
+
+
+def test_streams_are_lent_once_and_kept_by_role(monkeypatch):
+    import torch
+    from transportse_b200.batch import StreamShelf
+    made = []
+    monkeypatch.setattr(torch.cuda, "Stream", lambda device: made.append(device) or "s%d" % len(made))
+    shelf, dev = StreamShelf(), torch.device("cuda", 0)
+    a = shelf.take(dev, "step", 3)
+    b = shelf.take(dev, "step", 2)          # a is still lent
+    assert not set(a) & set(b) and len(made) == 5
+    shelf.give(dev, "step", b)
+    shelf.give(dev, "step", a)
+    assert shelf.take(dev, "step", 4) == a + b[:1] and len(made) == 5
+    assert shelf.take(dev, "build", 1) == ["s6"]                       # another role
+    assert shelf.take(torch.device("cuda", 1), "step", 1) == ["s7"]    # another device
+    shelf.give(dev, "step", shelf.take(dev, "step", 100))
+    assert sum(map(len, shelf.idle.values())) == StreamShelf.KEEP

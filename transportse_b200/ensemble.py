@@ -38,7 +38,7 @@ import numpy
 import torch
 
 from . import _native as N
-from .batch import BatchGate
+from .batch import SHELF, BatchGate
 from .driver import Simulation
 
 # resident cooperative blocks per SM of the mixed-precision sweep kernel
@@ -236,6 +236,18 @@ class Ensemble:
         apart (``setup_s``, ``step_s``, ``stepping_cell_updates_per_s``);
         otherwise models are admitted one by one as memory frees up and only
         the whole wall time is known.  Batched runs always prebuild."""
+        nthreads = len(self.configs) if self.batched else self.concurrency
+        # every model is set up on one stream: what one run's models free serves
+        # the next run's, whatever thread built them
+        built_on = SHELF.take(self.device, "build", 1)
+        stepped_on = SHELF.take(self.device, "step", nthreads)
+        try:
+            return self._run(steps, keep, prebuild, built_on[0], stepped_on)
+        finally:
+            SHELF.give(self.device, "build", built_on)
+            SHELF.give(self.device, "step", stepped_on)
+
+    def _run(self, steps, keep, prebuild, build_stream, step_streams):
         needs = [state_bytes(cfg, self.precision) for cfg in self.configs]
         if prebuild is None:
             prebuild = sum(needs) <= self.budget.total
@@ -255,8 +267,7 @@ class Ensemble:
                 todo.put(i)
 
             def builder():
-                stream = torch.cuda.Stream(device=self.device)
-                with torch.cuda.device(self.device), torch.cuda.stream(stream):
+                with torch.cuda.device(self.device), torch.cuda.stream(build_stream):
                     while True:
                         try:
                             i = todo.get_nowait()
@@ -268,7 +279,7 @@ class Ensemble:
                                                   self.cluster)
                         except Exception as e:
                             errors.append((i, e))
-                    stream.synchronize()
+                    build_stream.synchronize()
             ths = [threading.Thread(target=builder, daemon=True) for _ in range(min(8, n))]
             for th in ths:
                 th.start()
@@ -285,13 +296,11 @@ class Ensemble:
             todo = queue.Queue()
             for i in range(n):
                 todo.put(i)
-            nthreads = n if self.batched else self.concurrency
             if self.batched:
                 for _ in range(n):
                     self.gate.join()   # every model is a member before any solves
 
-            def stepper():
-                stream = torch.cuda.Stream(device=self.device)
+            def stepper(stream):
                 while True:
                     try:
                         i = todo.get_nowait()
@@ -303,16 +312,16 @@ class Ensemble:
                             stream.synchronize()
                     except Exception as e:   # reported after all workers stop
                         errors.append((i, e))
+                        stream.synchronize()
                     sims[i] = None   # its device memory goes back to the pool
 
-            threads = [threading.Thread(target=stepper, daemon=True) for _ in range(nthreads)]
+            threads = [threading.Thread(target=stepper, args=(st,), daemon=True) for st in step_streams]
         else:
             todo = queue.Queue()
             for i, cfg in enumerate(self.configs):
                 todo.put((i, cfg))
 
-            def admitter():
-                stream = torch.cuda.Stream(device=self.device)
+            def admitter(stream):
                 while True:
                     try:
                         i, cfg = todo.get_nowait()
@@ -330,7 +339,7 @@ class Ensemble:
                     finally:
                         self.budget.release(needs[i])
 
-            threads = [threading.Thread(target=admitter, daemon=True) for _ in range(self.concurrency)]
+            threads = [threading.Thread(target=admitter, args=(st,), daemon=True) for st in step_streams]
         t1 = time.perf_counter()
         for th in threads:
             th.start()
