@@ -175,3 +175,27 @@ def test_exact_solves_equal_the_streaming_kernels(shape, resident, cuda_device):
         out.append(got)
     _same(out[0], out[1])
     _same(out[0], out[2])
+
+
+# cells of a colour: one block's threads and one more pair, every SM's threads and more
+@pytest.mark.parametrize("shape", [(16, 16, 6), (16, 16, 8), (37, 96, 64), (111, 64, 32), (111, 64, 34), (5, 211, 431)])
+def test_plain_loads_ahead_of_the_barrier_equal_the_staged_kernel(shape, cuda_device):
+    """The plain-load FP64 kernel, whose threads load their first cell of the
+    next half-sweep before the barrier, against the staged one: convergence,
+    dt halvings, stops, omega < 1; and whichever of them the size selects."""
+    cfg, rng, args, P, BP, WP = _case(shape, 5)
+    C, D, one, z = rng.uniform(0, 1, shape), 1e-6 * rng.uniform(0.5, 1.5, shape), numpy.ones(shape), numpy.zeros(shape)
+    q = [rng.uniform(-1e-4, 1e-4, shape) for _ in range(3)]
+    m = model_for(cfg, cuda_device)
+    nk, out = NumpyKernels(m), []
+    for mode in (0, 1, 2):
+        m.sweep, got = mode, []
+        for max_it, min_dt in ((20000, 1e-8), (40, 1.0), (7, 400.0)):
+            got += [*nk.compute_P(P.copy(), *args, z, z, z, 3600.0, BP, WP, SOR=1.7, max_it=max_it, inc_it=1.25,
+                                  max_dt=1e5, min_dt=min_dt, P_conv=1e-10), m.last_status.halvings]
+        for omega in (1.0, 0.5, 0.0):
+            got += [*nk.compute_C(C.copy(), D, D, D, args[3], args[2], *q, 600.0, BP, WP, one, z, omega=omega, SOR=1.1,
+                                  max_it=100, inc_it=1.05, max_dt=1e5, min_dt=1e-8, C_conv=1e-11)]
+        out.append(got)
+    _same(out[0], out[1])
+    _same(out[0], out[2])

@@ -71,6 +71,10 @@ struct PressureForm {
         idx[n++] = PA_DEN;
         return n;
     }
+    // does update_with() read array k?
+    __device__ __forceinline__ bool reads(int k) const {
+        return k < PA_AB || k >= PA_RPN || (k < PA_IJ ? xgrav : zgrav) != 0;
+    }
     static constexpr int kSolution = PA_P;
     static constexpr int kDen = PA_DEN, kRhs = PA_RPN;
     // The resident solve's arrays of a group, in a fixed order for either
@@ -174,6 +178,10 @@ struct TransportForm {
         if (useEX) idx[n++] = TA_EX;
         idx[n++] = TA_DEN;
         return n;
+    }
+    // does update_with() read array k?
+    __device__ __forceinline__ bool reads(int k) const {
+        return k == TA_Y ? useY != 0 : k == TA_EX ? useEX != 0 : true;
     }
     static constexpr int kSolution = TA_X;
     static constexpr int kDen = TA_DEN, kRhs = TA_RXN;

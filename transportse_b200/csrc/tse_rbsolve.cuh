@@ -26,7 +26,7 @@ struct SolveCtl {
     int max_it;
     int pressure_schedule;      // 1: L2 every it below 50, then every 10th
     int stop_on_first;          // 1: converged after one it (omega == 0)
-    int plain_sweep;            // 1: plain-load kernel even where the staged one fits
+    int plain_sweep;            // 1: plain-load kernel even where the staged one fits (plain_sweep())
     double* X[2];               // solution per colour
     const uint8_t* mask[2];
     double* partials;           // 2 doubles per block
@@ -36,9 +36,40 @@ struct SolveCtl {
 
 constexpr int kMaxBlocks = 16384;
 
+// One block a SM (148 arrivals a barrier) of as many threads as registers last
+// for, a cell a thread where that covers the grid.  Bound: latency, of the
+// barrier and of the loads behind it; what a thread's first cell reads, but for
+// the neighbours, is loaded before the barrier.  us an iteration on a B200
+// (pressure, x and z buoyancy): 72^3 16.0 -> 12.9, 80^3 16.3 -> 14.8, 100^3 31.4 ->
+// 27.6; 512 or 640 threads 12.5, 14.4 and from 96^3 on a tenth more, 1024 (which
+// spills) 14.4 at 72^3.
+constexpr int kPlainBlock = 768;
+// From this many cells of a colour on the staged sweep (tse_rbsolve_tma.cuh) is
+// the faster one, below this one (staged / plain: 72^3 19.3 / 12.9, 100^3 30.2 /
+// 27.6, 110^3 35.8 / 33.4, 128 x 128 x 127 47.1 / 46.4, 192 x 160 x 101 65.1 / 74.4).
+constexpr long long kStagedMinNc = 1000000;
+
+// `sweep` as the entry points take it: 1 plain, 2 staged, else by size
+inline int plain_sweep(int sweep, const Layout& L) { return sweep == 1 || (sweep != 2 && L.Nc < kStagedMinNc); }
+
+// What the update of a cell reads that the other colour does not write.
 template <class Form>
-__global__ void __launch_bounds__(kBlock, 3) rb_solve_kernel(Form F, SolveCtl c) {
-    __shared__ double sh[kBlock / 32];
+struct Ahead {
+    double a[Form::kCoef], xold;
+    uint8_t f;
+    __device__ __forceinline__ void load(const Form& F, const SolveCtl& c, int col, long long m) {
+        const double* b = (col ? F.arr[1] : F.arr[0]) + m;
+        f = (col ? c.mask[1] : c.mask[0])[m];
+        xold = (col ? c.X[1] : c.X[0])[m];
+#pragma unroll
+        for (int k = 0; k < Form::kCoef; ++k)
+            if (F.reads(k)) a[k] = b[(long long)k * F.Ncal];
+    }
+};
+
+template <class Form>
+__global__ void __launch_bounds__(kPlainBlock, 1) rb_solve_kernel(Form F, SolveCtl c) {
+    __shared__ double sh[kPlainBlock / 32];
     __shared__ double s_diff;
     const unsigned nb = gridDim.x;
     const long long tid0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -49,30 +80,38 @@ __global__ void __launch_bounds__(kBlock, 3) rb_solve_kernel(Form F, SolveCtl c)
     double t = 0.0, dt = c.dt, diff = 1e100;
     int converged = 0, num_it = 0, num_sub_it = 0, halvings = 0, err = 0, nev = 0;
 
+    Ahead<Form> own;
+    if (tid0 < Nc) own.load(F, c, 0, tid0);
     while (!converged) {
         num_it += 1;
         num_sub_it += 1;
         double d2 = 0.0, o2 = 0.0;
         const bool check = c.pressure_schedule ? (num_it < 50 || num_it % 10 == 0) : true;
         for (int col = 0; col < 2; ++col) {
-            double* Xw = c.X[col];
-            const double* Xo = c.X[1 - col];
-            const uint8_t* msk = c.mask[col];
+            double* Xw = col ? c.X[1] : c.X[0];
+            const double* Xo = col ? c.X[0] : c.X[1];
             for (long long m = tid0; m < Nc; m += stride) {
-                const uint8_t f = msk[m];
-                const double xold = Xw[m];
+                if (m != tid0) own.load(F, c, col, m);
+                const uint8_t f = own.f;
+                const double xold = own.xold;
                 o2 = o2 + xold * xold;
                 if (f & F_ACTIVE) {
-                    const double xn = F.update(col, m, f, xold, Xo);
+                    const long long zo = f >> 7;
+                    const double xn = F.update_with(
+                        [&](int k) { return own.a[k]; },
+                        [&](int q) { return __ldcg(Xo + m + nb_offset(q, F.SX, F.H, zo)); }, f, xold);
                     Xw[m] = xn;
                     const double d = xn - xold;
                     d2 = d2 + d * d;
                 }
             }
+            // the first cell's loads of the next half-sweep pass behind the
+            // barrier: all of them were last written by this thread
+            if (tid0 < Nc) own.load(F, c, col ^ 1, tid0);
             if (col == 1 && check) {
                 // per-block partial sums, published by the barrier below
-                double b1 = block_sum<kBlock>(d2, sh);
-                double b2 = block_sum<kBlock>(o2, sh);
+                double b1 = block_sum<kPlainBlock>(d2, sh);
+                double b2 = block_sum<kPlainBlock>(o2, sh);
                 if (threadIdx.x == 0) {
                     c.partials[2 * blockIdx.x] = b1;
                     c.partials[2 * blockIdx.x + 1] = b2;
@@ -88,8 +127,8 @@ __global__ void __launch_bounds__(kBlock, 3) rb_solve_kernel(Form F, SolveCtl c)
                 s1 = s1 + __ldcg(c.partials + 2 * b);
                 s2 = s2 + __ldcg(c.partials + 2 * b + 1);
             }
-            s1 = block_sum<kBlock>(s1, sh);
-            s2 = block_sum<kBlock>(s2, sh);
+            s1 = block_sum<kPlainBlock>(s1, sh);
+            s2 = block_sum<kPlainBlock>(s2, sh);
             if (threadIdx.x == 0) {
                 double l2 = sqrt(s1) / sqrt(s2 + 1e-200);
                 s_diff = (l2 != l2) ? 1.0 : l2;
@@ -117,6 +156,7 @@ __global__ void __launch_bounds__(kBlock, 3) rb_solve_kernel(Form F, SolveCtl c)
                 halvings += 1;
                 for (int col = 0; col < 2; ++col)
                     for (long long m = tid0; m < Nc; m += stride) F.reassemble(col, m, dt);
+                if (tid0 < Nc) own.load(F, c, 0, tid0);
                 if (!grid_sync(c.bar, nb)) { err = 1; break; }
             }
             if (dt <= c.min_dt) break;
@@ -140,24 +180,16 @@ __global__ void __launch_bounds__(kBlock, 3) rb_solve_kernel(Form F, SolveCtl c)
 // Launch the persistent loop with as many co-resident blocks as useful.
 template <class Form>
 inline int launch_rb_solve(const Form& F, SolveCtl& ctl, cudaStream_t stream) {
-    static int cached_dev = -1, cached_per_sm = 0, cached_sms = 0;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev != cached_dev) {
-        cudaDeviceGetAttribute(&cached_sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cached_per_sm, rb_solve_kernel<Form>,
-                                                      kBlock, 0);
-        cached_dev = dev;
-    }
-    long long maxb = (long long)cached_sms * (cached_per_sm > 0 ? cached_per_sm : 1);
-    // at least 4 cells per thread per half-sweep, at most the co-resident set
-    long long want = (ctl.L.Nc + (long long)kBlock * 4 - 1) / ((long long)kBlock * 4);
-    if (want < 1) want = 1;
-    long long nb = want < maxb ? want : maxb;
-    if (nb > kMaxBlocks) nb = kMaxBlocks;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return TSE_ERR_LAUNCH;
+    // a cell a thread, at most the co-resident blocks
+    const long long want = (ctl.L.Nc + kPlainBlock - 1) / kPlainBlock;
+    const long long nb = want < 1 ? 1 : want < sms ? want : sms;
     void* args[] = {(void*)&F, (void*)&ctl};
     cudaError_t e = cudaLaunchCooperativeKernel((const void*)rb_solve_kernel<Form>, dim3((unsigned)nb),
-                                                dim3(kBlock), args, 0, stream);
+                                                dim3(kPlainBlock), args, 0, stream);
     return e == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
 }
 
