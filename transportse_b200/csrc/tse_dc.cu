@@ -32,6 +32,7 @@
 // L2 -- against 89 bytes of coefficients and flags for the FP64 form.
 //
 // Compiled with FMA contraction (no bit-exactness is claimed for this form).
+#include <cstddef>
 #include <type_traits>
 
 #include "tse_dc.cuh"
@@ -173,9 +174,12 @@ __global__ void __launch_bounds__(kBlock) dc_apply_residual_kernel(Form F, DcCtl
     if (threadIdx.x == 0) c.partials[blockIdx.x] = s2;
 }
 
-// x^2 total into the state; counts the cycle
-__global__ void dc_x2_kernel(DcCtl c, int nparts) {
+// x^2 total into the state; counts the cycle; zero_prog: the staged sweep's
+// counters start at 0 (a memset of their own costs 4 us a cycle)
+__global__ void dc_x2_kernel(DcCtl c, int nparts, int zero_prog = 0) {
     __shared__ double sh[kBlock / 32];
+    if (zero_prog)
+        for (int q = threadIdx.x; q < (int)(kProgBytes / sizeof(unsigned)); q += kBlock) c.prog[q] = 0;
     double s = 0.0;
     int b = threadIdx.x;
     // eight loads in flight, summed in the order of the plain loop
@@ -865,20 +869,15 @@ static int run_dc(SolveSetup<Form>& S, double dt, double inc_it, double max_dt, 
     bool final_apply = false;
     for (;;) {
         if (first_parts > 0) {
-            dc_x2_kernel<<<1, kBlock, 0, stream>>>(c, first_parts);
+            dc_x2_kernel<<<1, kBlock, 0, stream>>>(c, first_parts, nb_tma > 0);
             first_parts = 0;
         } else {
             const unsigned rb = (unsigned)res_blocks(S.L.Nc);
             dc_residual_kernel<<<rb, kBlock, 0, stream>>>(S.F, c);
-            dc_x2_kernel<<<1, kBlock, 0, stream>>>(c, (int)rb);
+            dc_x2_kernel<<<1, kBlock, 0, stream>>>(c, (int)rb, nb_tma > 0);
         }
         void* args[] = {(void*)&c};
         void* targs[] = {(void*)&c, (void*)&T};
-        // staged sweep: its counters start at 0
-        if (nb_tma > 0 && cudaMemsetAsync(c.prog, 0, kProgBytes, stream) != cudaSuccess) {
-            rc = TSE_ERR_LAUNCH;
-            break;
-        }
         if (timing) cudaEventRecord(ev0, stream);
         if (cudaGetLastError() != cudaSuccess) {
             rc = TSE_ERR_LAUNCH;
@@ -894,24 +893,30 @@ static int run_dc(SolveSetup<Form>& S, double dt, double inc_it, double max_dt, 
             break;
         }
         if (timing) cudaEventRecord(ev1, stream);
-        int head[2] = {EV_ERROR, 0};   // event, num_it
-        if (cudaMemcpyAsync(&head[0], &c.st->event, sizeof(int), cudaMemcpyDeviceToHost, stream) !=
-                cudaSuccess ||
-            cudaMemcpyAsync(&head[1], &c.st->num_it, sizeof(int), cudaMemcpyDeviceToHost, stream) !=
+        // one read of the scalars (a pageable copy waits for the stream anyway)
+        struct {
+            double t, dt, diff, x2;
+            int num_it, num_sub_it, halvings, converged, event;
+        } head;
+        static_assert(offsetof(DcState, event) == offsetof(decltype(head), event) &&
+                          offsetof(DcState, num_it) == offsetof(decltype(head), num_it) &&
+                          offsetof(DcState, dt) == offsetof(decltype(head), dt),
+                      "DcState begins like this");
+        if (cudaMemcpyAsync(&head, c.st, offsetof(DcState, event) + sizeof(int), cudaMemcpyDeviceToHost, stream) !=
                 cudaSuccess ||
             cudaStreamSynchronize(stream) != cudaSuccess) {
             rc = TSE_ERR_LAUNCH;
             break;
         }
-        const int event = head[0];
+        const int event = head.event;
         if (timing) {
             float ms = 0.0f;
             cudaEventElapsedTime(&ms, ev0, ev1);
             opts->sweep_launches += 1;
-            opts->sweep_iterations += head[1] - prev_it;
+            opts->sweep_iterations += head.num_it - prev_it;
             opts->sweep_ms += ms;
         }
-        prev_it = head[1];
+        prev_it = head.num_it;
         if (S.lean && event == EV_STOP_HALVED) {
             // the caller's field still holds the entry state
             dc_status_kernel<<<1, 1, 0, stream>>>(c.st, d_status);
@@ -922,11 +927,8 @@ static int run_dc(SolveSetup<Form>& S, double dt, double inc_it, double max_dt, 
             return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
         }
         if (S.lean && event == EV_HALVE) {
-            double half = 0.0;
-            if (cudaMemcpyAsync(&half, &c.st->dt, sizeof(double), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
-                cudaStreamSynchronize(stream) != cudaSuccess ||
-                cudaMemsetAsync(dbase, 0, (size_t)2 * dlen * sizeof(float), stream) != cudaSuccess ||
-                again(half, &first_parts) != TSE_OK) {
+            if (cudaMemsetAsync(dbase, 0, (size_t)2 * dlen * sizeof(float), stream) != cudaSuccess ||
+                again(head.dt, &first_parts) != TSE_OK) {
                 rc = TSE_ERR_LAUNCH;
                 break;
             }

@@ -107,11 +107,6 @@ struct PressureForm {
     __device__ __forceinline__ double k(int col, long long m, int q) const {
         return arr[col][(PA_A + q) * Ncal + m];
     }
-    __device__ __forceinline__ double update(int col, long long m, uint8_t f, double xold,
-                                             const double* Xo) const {
-        const double s = sum(col, m, f, Xo);
-        return (1.0 - SOR) * xold + (SOR * s) / den(col, m);
-    }
     template <class A, class X>
     __device__ __forceinline__ double update_with(A a, X x, uint8_t f, double xold) const {
         const double s = sum_with(a, x, f);
@@ -216,11 +211,6 @@ struct TransportForm {
     // coefficient of neighbour q in sum(): omega * (upwinded coefficient)
     __device__ __forceinline__ double k(int col, long long m, int q) const {
         return omega * arr[col][(TA_A + q) * Ncal + m];
-    }
-    __device__ __forceinline__ double update(int col, long long m, uint8_t f, double xold,
-                                             const double* Xo) const {
-        const double num = sum(col, m, f, Xo);
-        return (1.0 - SOR) * xold + (SOR * num) / den(col, m);
     }
     template <class A, class X>
     __device__ __forceinline__ double update_with(A a, X x, uint8_t f, double xold) const {
