@@ -88,7 +88,8 @@ typedef struct TsePressureArgs {
     int32_t max_it;
     int32_t sweep;    /* FP64 solves' sweep kernel for this call (no counterpart
                          in the reference): 0 (default) the resident kernel
-                         where the grid's state fits on the chip, else as 2;
+                         where the grid's state fits on the chip, else plain
+                         loads below a million cells of a colour, else as 2;
                          1 plain loads; 2 the bulk-copy staged kernel wherever
                          its stages fit, else plain loads.  Same cell values
                          either way.  The mixed-precision forms ignore it. */

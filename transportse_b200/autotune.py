@@ -2,7 +2,8 @@
 
 The mixed-precision solves spend nearly all their time in one kernel, the
 bulk-copy staged red-black sweep (``dc_sweep_tma_kernel``).  Its shape is a
-compile-time choice among 18 instances:
+compile-time choice (or, for a grid that fits on the chip, the resident solve's
+single launch):
 
 * chunk -- cells a producer copies and a consumer group relaxes at a time
   (256, 512, 1024): larger chunks issue fewer, larger copies, smaller ones

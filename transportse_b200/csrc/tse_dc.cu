@@ -16,8 +16,9 @@
 // FP32 resolves d to ~6e-8 |d|, so the measured change stays ~1e3 times above
 // d's rounding and the iteration counts track the FP64 form's.
 //
-// Kernels: the FP32 sweeps run in one cooperative kernel that iterates until
-// an event (converged, cycle end, dt halving, stop): dc_sweep_tma_kernel,
+// Kernels: a grid that fits on the chip solves in one launch, cycles included
+// (dc_resident_kernel, tse_dc_resident.cuh).  Else the FP32 sweeps run in one
+// cooperative kernel that iterates until an event (converged, cycle end, dt halving, stop): dc_sweep_tma_kernel,
 // which stages each chunk's data in shared memory with bulk asynchronous
 // copies, or, where its stages do not fit, dc_sweep_kernel (48 registers,
 // 5 blocks per SM, plain loads).  The FP64 residual, the x += d update and the dt

@@ -190,7 +190,8 @@ __device__ __forceinline__ double mobility(double dsum, const Perm& a, const Per
 
 // 255 x 256 x 127 (B200): 418 us with a thread a cell and the operator's
 // divisions, 265 now (10 arrays, 101 us); a tenth more with 2 or 3 blocks a SM or
-// with 5.  Bound: FP64 arithmetic, 15 reciprocals and 23 quotients a cell.
+// with 5.  Bound: 15 reciprocals and 23 quotients a cell and the loads' latency
+// (FP64 pipe 42 % busy, 28 warps a SM, DRAM 30 %).
 __global__ void __launch_bounds__(kBlock, kWalkBlocksQ)
     compute_q_kernel(TseGrid g, Walk w, const double* P, const double* BP, const double* Kx, const double* Ky,
                      const double* Kz, double* qx, double* qy, double* qz, const double* nue,
@@ -313,7 +314,8 @@ __device__ __forceinline__ double harm_of(double dsum, double a1, double a2, boo
 
 // A face's mean density is the same bits from either side.  255 x 256 x 127
 // (B200): 305 us before, 190 now (11 arrays, 112 us); a tenth more with 2 blocks a SM
-// or with 4.  Bound: FP64 arithmetic, 7 reciprocals and 18 quotients a cell.
+// or with 4.  Bound: 7 reciprocals and 18 quotients a cell and the loads'
+// latency (FP64 pipe 41 % busy, 21 warps a SM, DRAM 45 %).
 __global__ void __launch_bounds__(kBlock, kWalkBlocksE)
     flow_error_kernel(TseGrid g, Walk w, const double* P, const double* Pn, const double* qx, const double* qy,
                       const double* qz, const double* WP, const double* phi, const double* c_f,

@@ -390,10 +390,11 @@ struct HeatKind {
     }
 };
 
-// Both assemblies are bound by the latency of their loads (15 input arrays,
-// neighbours included).  Four 256-thread blocks per SM (64 registers, some
-// spilled): with the face values read from the face pass, measured on the
-// 256 x 256 x 128 reservoir (whole calls, one box, one call each), a species
+// The exact form's assemblies are bound by the latency of their loads (15 input
+// arrays, neighbours included).  Four 256-thread blocks per SM (64 registers,
+// some spilled): with the face values read from the face pass, measured on the
+// 256 x 256 x 128 reservoir (whole mixed-precision calls, which shared these
+// kernels), a species
 // solve of 5 iterations took 1.65 ms at four blocks, 1.89 at three and 2.09 at
 // two (heat, 3 iterations: 1.39, 1.51, 1.65 ms).
 #ifndef TSE_ASM_MINB
