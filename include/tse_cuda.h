@@ -425,6 +425,12 @@ int32_t tse_mass_totals(const TseGrid *grid, const double *phi,
 int32_t tse_selftest_bounded_waits(int32_t *d_result, double timeout_s, void *d_ws,
                                    size_t ws_bytes, void *stream);
 
+/* The same for the resident solves' waits and the overlapped sweep's (limit at
+ * most 1 s): d_result[0] an edge record and [1] a sum record nobody writes, [2]
+ * a report nobody makes.  d_ws: 32 KB of device memory. */
+int32_t tse_selftest_resident_waits(int32_t *d_result, double timeout_s, void *d_ws,
+                                    size_t ws_bytes, void *stream);
+
 /* Batched solves run so far by the fused form's device-driven loop and by its
  * host loop (TseDcOptions.host_loop; no counterpart in the reference). */
 int32_t tse_batch_loop_stats(int64_t *graph_solves, int64_t *host_solves);

@@ -138,6 +138,7 @@ SIGNATURES = {
     "tse_mass_totals": (_I, [_G, _P, _P, _P, _PP, _PP, _I, _P, _P, _P, _P, _P, _P, _P, _P, _S,
                              _P]),
     "tse_selftest_bounded_waits": (_I, [_P, _D, _P, _S, _P]),
+    "tse_selftest_resident_waits": (_I, [_P, _D, _P, _S, _P]),
     "tse_batch_loop_stats": (_I, [ct.POINTER(ct.c_int64), ct.POINTER(ct.c_int64)]),
     "tse_version": (ct.c_char_p, []),
 }

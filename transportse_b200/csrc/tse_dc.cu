@@ -365,24 +365,6 @@ __global__ void __launch_bounds__(kSweepBlock, kSweepMinBlocks) dc_sweep_kernel(
 // 192 x 128 26.2 -> 23.3, 256 x 256 x 128 42.0-42.8 -> 39.7-42.3 (0.94 of the
 // measured HBM rate at best), 320 x 320 x 160 88.3 -> 82.6-83.5; with the record
 // blocks and 8 or 16 consumer warps 13.5, 22.2, 38.8-41.2 and 83.4-86.
-// seg_wait: a report's count has reached `target` (acquire); bounded.
-__device__ __forceinline__ bool seg_wait(const unsigned* count, unsigned target, GridBarrier* bar,
-                                         volatile int* err) {
-    if ((int)(ld_acquire_u32(count) - target) >= 0) return true;
-    const uint64_t t0 = globaltimer();
-    unsigned spins = 0;
-    while ((int)(ld_acquire_u32(count) - target) < 0) {
-        if ((++spins & 63u) == 0u &&
-            (*err || *(volatile int*)&bar->error || globaltimer() - t0 > kBarrierTimeoutNs)) {
-            *err = 1;
-            atomicExch(&bar->error, 1);
-            return false;
-        }
-        __nanosleep(32);
-    }
-    return true;
-}
-
 template <int RING, int PIPES, int CHUNK, bool WIDE>
 __global__ void __launch_bounds__(DcLayout<PIPES, WIDE>::kThreads, DcLayout<PIPES, WIDE>::kMinBlocks)
     dc_sweep_tma_kernel(DcCtl c, TmaStage T) {

@@ -332,6 +332,23 @@ constexpr int kSegs = 2;
 constexpr int kSegWords = 8, kSegBase = 32;
 constexpr size_t kProgBytes = (kSegBase + kSegs * kSegWords) * sizeof(unsigned);
 
+// a report's count has reached `target` (acquire); bounded
+__device__ __forceinline__ bool seg_wait(const unsigned* count, unsigned target, GridBarrier* bar, volatile int* err,
+                                         unsigned long long timeout_ns = kBarrierTimeoutNs) {
+    if ((int)(ld_acquire_u32(count) - target) >= 0) return true;
+    const uint64_t t0 = globaltimer();
+    unsigned spins = 0;
+    while ((int)(ld_acquire_u32(count) - target) < 0) {
+        if ((++spins & 63u) == 0u &&
+            (*err || *(volatile int*)&bar->error || globaltimer() - t0 > timeout_ns)) {
+            *err = 1;
+            atomicExch(&bar->error, 1);
+            return false;
+        }
+        __nanosleep(32);
+    }
+    return true;
+}
 
 __host__ __device__ inline TmaStage tma_stage(int H, int C = kTmaChunk) {
     TmaStage t;

@@ -229,11 +229,12 @@ struct ResWait {
     volatile int* err;
     unsigned tries;
     uint64_t t0;
+    unsigned long long timeout_ns;
     __device__ __forceinline__ bool go_on() {
         if ((++tries & 255u) != 0u) return true;
         const uint64_t now = globaltimer();
         if (tries == 256u) t0 = now;
-        if (*err || *(volatile int*)&bar->error || now - t0 > kBarrierTimeoutNs) {
+        if (*err || *(volatile int*)&bar->error || now - t0 > timeout_ns) {
             *err = 1;
             atomicExch(&bar->error, 1);
             return false;
@@ -248,11 +249,12 @@ struct ResWait {
 template <int NT>
 __device__ __forceinline__ void res_poll(const uint64_t* recs, int plane, unsigned tag, uint4* s,
                                          const int* hrec, const unsigned short* hp, int nh, GridBarrier* bar,
-                                         volatile int* err) {
+                                         volatile int* err,
+                                         unsigned long long timeout_ns = kBarrierTimeoutNs) {
     for (int h = threadIdx.x; h < nh; h += NT) {
         const uint64_t* r = recs + 2 * hrec[h];
         uint64_t a, b, c, d;
-        ResWait wt = {bar, err, 0u, 0};
+        ResWait wt = {bar, err, 0u, 0, timeout_ns};
         for (;;) {
             ld_words2(r, a, b);
             ld_words2(r + plane, c, d);
@@ -329,8 +331,8 @@ struct ResPeers {
 // kResCopies records, which the other blocks poll (all blocks polling all
 // records kept the memory's few hot sectors so busy that a sum took 7 us at
 // 148 blocks).  Two sets of records alternate with `count`, tagged with count
-// + 1.  Contains block barriers; a caller has one between two calls.  False
-// when a wait ran out.
+// + 1.  Contains block barriers; a caller has one between two calls.  False, in
+// all of a block's threads, when a wait of this block ran out here or before.
 constexpr int kResCopies = 8;
 constexpr int kResSetWords = kResMaxBlocks * 4 + kResCopies * 16;   // copies on lines of their own
 struct ResSumShared {
@@ -340,8 +342,9 @@ struct ResSumShared {
 };
 
 __device__ __forceinline__ bool res_poll_pair(const uint64_t* s, unsigned tag, double& A, double& B,
-                                              GridBarrier* bar, volatile int* err) {
-    ResWait wt = {bar, err, 0u, 0};
+                                              GridBarrier* bar, volatile int* err,
+                                              unsigned long long timeout_ns = kBarrierTimeoutNs) {
+    ResWait wt = {bar, err, 0u, 0, timeout_ns};
     uint64_t v0, v1, v2, v3;
     for (;;) {
         ld_words2(s, v0, v1);
@@ -364,7 +367,8 @@ __device__ __forceinline__ void res_write_pair(uint64_t* s, unsigned tag, double
 template <int NT, int MODE>
 __device__ __forceinline__ bool res_team_sum(double& va, double& vb, ResSumShared& sh, uint64_t* slots,
                                              unsigned nb, unsigned b, unsigned count, GridBarrier* bar,
-                                             volatile int* err) {
+                                             volatile int* err,
+                                             unsigned long long timeout_ns = kBarrierTimeoutNs) {
     constexpr int NW = NT / 32;
     static_assert(NT <= kResMaxThreads && NT >= kResMaxBlocks && NW <= 32, "one polling thread a block");
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -422,7 +426,7 @@ __device__ __forceinline__ bool res_team_sum(double& va, double& vb, ResSumShare
     if (b != 0) {
         if (threadIdx.x == 0) {
             res_write_pair(set + 4 * b, tag, A, B);
-            res_poll_pair(copies + 16 * (b % kResCopies), tag, A, B, bar, err);
+            res_poll_pair(copies + 16 * (b % kResCopies), tag, A, B, bar, err, timeout_ns);
             sh.total[0] = A;
             sh.total[1] = B;
         }
@@ -435,7 +439,7 @@ __device__ __forceinline__ bool res_team_sum(double& va, double& vb, ResSumShare
             x = A;
             y = B;
         } else if (q < nb) {
-            res_poll_pair(set + 4 * q, tag, x, y, bar, err);
+            res_poll_pair(set + 4 * q, tag, x, y, bar, err, timeout_ns);
         }
         if ((q & ~31u) < nb) {
 #pragma unroll
@@ -462,10 +466,10 @@ __device__ __forceinline__ bool res_team_sum(double& va, double& vb, ResSumShare
             }
         }
     }
-    __syncthreads();
+    const bool ok = __syncthreads_and(*err == 0);   // the same for all threads
     va = sh.total[0];
     vb = sh.total[1];
-    return *err == 0;
+    return ok;
 }
 
 // A launch's exchange memory: a counter, the sum slots, and per colour one

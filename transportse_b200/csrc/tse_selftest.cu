@@ -1,12 +1,15 @@
-// Self-test of the bounded waits every persistent kernel of the library
-// relies on.  Each case runs one wait whose condition nothing ever makes true
-// -- a grid barrier that counts one block more than the launch has, a
-// counter barrier with an unreachable target, an mbarrier no one arrives at
-// -- and records whether the wait gave up after its time limit and raised its
-// error flag, as it must for a solver kernel to return
-// TSE_STATUS_BARRIER_TIMEOUT instead of holding the GPU.  Nothing faults: the
-// kernels only wait, give up and return.
+// Self-tests of what the kernels rely on and no solve can show.
+//
+// Bounded waits of every persistent kernel of the library.  Each case runs one
+// wait whose condition nothing ever makes true -- a grid barrier that counts one
+// block more than the launch has, a counter barrier with an unreachable target,
+// an mbarrier no one arrives at, a record or a report no one writes -- and
+// records whether the wait gave up after its time limit and raised its error
+// flag, as it must for a solver kernel to return TSE_STATUS_BARRIER_TIMEOUT
+// instead of holding the GPU.  Nothing faults: the kernels only wait, give up
+// and return.
 #include "tse_dc.cuh"
+#include "tse_resident.cuh"
 
 namespace tse {
 
@@ -41,6 +44,42 @@ __global__ void __launch_bounds__(128) selftest_wait_kernel(int which, GridBarri
     }
 }
 
+// The resident solves' waits: an edge record and a sum record nobody writes
+// (result[0], result[1]: gave up, flags raised).
+__global__ void __launch_bounds__(kResMaxThreads) selftest_resident_kernel(int which, GridBarrier* bar,
+                                                                           uint64_t* words, int* result,
+                                                                           unsigned long long timeout_ns) {
+    __shared__ uint4 ring[1];
+    __shared__ int hrec[1], s_err;
+    __shared__ unsigned short hp[1];
+    volatile int* err = &s_err;
+    uint64_t* slots = words + 4;   // words 0 .. 3: one edge record, never written
+    if (threadIdx.x == 0) {
+        s_err = 0;
+        hrec[0] = 0;
+        hp[0] = 0;
+    }
+    __syncthreads();
+    if (which == 0) {
+        res_poll<kResMaxThreads>(words, 2, 1u, ring, hrec, hp, 1, bar, err, timeout_ns);
+        __syncthreads();
+        if (threadIdx.x == 0) result[0] = *err && *(volatile int*)&bar->error;
+    } else if (threadIdx.x == 0) {
+        double A = 0.0, B = 0.0;
+        const bool ok = res_poll_pair(slots, 1u, A, B, bar, err, timeout_ns);
+        result[1] = !ok && *err && *(volatile int*)&bar->error;
+    }
+}
+
+// The staged sweep's wait for other blocks' reports
+__global__ void selftest_report_kernel(GridBarrier* bar, unsigned* counter, int* result,
+                                       unsigned long long timeout_ns) {
+    __shared__ int s_err;
+    s_err = 0;
+    const bool ok = seg_wait(counter, 1u, bar, (volatile int*)&s_err, timeout_ns);
+    *result = !ok && s_err && *(volatile int*)&bar->error;
+}
+
 }  // namespace tse
 
 using namespace tse;
@@ -67,6 +106,31 @@ extern "C" int32_t tse_selftest_bounded_waits(int32_t* d_result, double timeout_
                       : cudaLaunchKernel((const void*)selftest_wait_kernel, dim3(1), dim3(128), args, 0,
                                          stream);
         if (e != cudaSuccess) return TSE_ERR_LAUNCH;
+    }
+    return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
+}
+
+extern "C" int32_t tse_selftest_resident_waits(int32_t* d_result, double timeout_s, void* d_ws, size_t ws_bytes,
+                                               void* stream_) {
+    const size_t words = 4 * sizeof(uint64_t) + kResSlotBytes, need = 512 + words;
+    if (!d_result || !d_ws || ws_bytes < need || !(timeout_s > 0.0)) return TSE_ERR_ARG;
+    if (timeout_s > 1.0) timeout_s = 1.0;
+    unsigned long long ns = (unsigned long long)(timeout_s * 1e9);
+    cudaStream_t stream = (cudaStream_t)stream_;
+    GridBarrier* bar = (GridBarrier*)d_ws;
+    unsigned* counter = (unsigned*)((char*)d_ws + 256);
+    uint64_t* w = (uint64_t*)((char*)d_ws + 512);
+    int* result = (int*)d_result;
+    if (cudaMemsetAsync(d_result, 0, 3 * sizeof(int32_t), stream) != cudaSuccess) return TSE_ERR_LAUNCH;
+    for (int which = 0; which < 3; ++which) {
+        if (cudaMemsetAsync(d_ws, 0, need, stream) != cudaSuccess) return TSE_ERR_LAUNCH;
+        if (which == 2) {
+            selftest_report_kernel<<<1, 1, 0, stream>>>(bar, counter, result + 2, ns);
+            continue;
+        }
+        void* args[] = {(void*)&which, (void*)&bar, (void*)&w, (void*)&result, (void*)&ns};
+        if (cudaLaunchCooperativeKernel((const void*)selftest_resident_kernel, dim3(1), dim3(kResMaxThreads), args, 0, stream) != cudaSuccess)
+            return TSE_ERR_LAUNCH;
     }
     return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
 }
