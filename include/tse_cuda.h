@@ -426,8 +426,11 @@ int32_t tse_selftest_bounded_waits(int32_t *d_result, double timeout_s, void *d_
                                    size_t ws_bytes, void *stream);
 
 /* The same for the resident solves' waits and the overlapped sweep's (limit at
- * most 1 s): d_result[0] an edge record and [1] a sum record nobody writes, [2]
- * a report nobody makes.  d_ws: 32 KB of device memory. */
+ * most 1 s): d_result[0] an edge record and [1] a sum record nobody writes, [4]
+ * a report nobody makes: 1 if the wait gave up and raised its flags.  A solve
+ * of two blocks that one leaves early: [2] 1 if the other block's sum was good
+ * all the same, [3] 1 if the last block to leave says that it failed.  d_ws: 32 KB of device
+ * memory.  Takes about 6 * timeout_s. */
 int32_t tse_selftest_resident_waits(int32_t *d_result, double timeout_s, void *d_ws,
                                     size_t ws_bytes, void *stream);
 

@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(NT, 1)
             bool refresh = false;
             if (check) {
                 double a = (double)d2, e = (double)dd;
-                // a poll that ran out shows here: no solve ends unchecked
+                // a poll of this block that ran out shows here
                 ok = res_team_sum<NT, MODE>(a, e, sum, w.mem.slots, nb, b, sums++, c.bar, err);
                 if (!ok) break;
                 const double ra = sqrt(a), l2 = ra / rx2;
@@ -305,16 +305,17 @@ __global__ void __launch_bounds__(NT, 1)
         cycles += 1;
         __syncthreads();
     }
-    if (leader) {
+    bool failed = event == EV_ERROR;
+    if (res_last<MODE>(w.mem.leavers, nb, b, failed)) {
         TseSolveStatus* s = status;
         s->t = t;
         s->dt = dt;
         s->diff = diff;
-        s->converged = event == EV_CONVERGED;
+        s->converged = event == EV_CONVERGED && !failed;
         s->num_it = num_it;
         s->num_sub_it = num_sub_it;
         s->halvings = halvings;
-        s->error = event == EV_ERROR ? TSE_STATUS_BARRIER_TIMEOUT : TSE_STATUS_OK;
+        s->error = failed ? TSE_STATUS_BARRIER_TIMEOUT : TSE_STATUS_OK;
         s->n_events = nev < 8 ? nev : 8;
         s->cycles = cycles;
     }

@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kXResThreads, 1)
                                        rbase, ++tag, peers, dxp, dyp, check, d2, o2);
             diff = 1e100;
             if (check) {
-                // a poll that ran out shows here: no solve ends unchecked
+                // a poll of this block that ran out shows here
                 ok = res_team_sum<NT, MODE>(d2, o2, sum, w.mem.slots, nb, b, sums++, c.bar, err);
                 if (!ok) break;
                 const double l2 = sqrt(d2) / sqrt(o2 + 1e-200);
@@ -270,16 +270,17 @@ __global__ void __launch_bounds__(kXResThreads, 1)
             if (!count_sync(w.mem.counter, ++bars * nb, c.bar)) { fail = 1; break; }
         }
     }
-    if (leader) {
+    bool failed = fail != 0;
+    if (res_last<MODE>(w.mem.leavers, nb, b, failed)) {
         TseSolveStatus* s = c.status;
         s->t = t;
         s->dt = dt;
         s->diff = diff;
-        s->converged = converged;
+        s->converged = converged && !failed;
         s->num_it = num_it;
         s->num_sub_it = num_sub_it;
         s->halvings = halvings;
-        s->error = fail ? TSE_STATUS_BARRIER_TIMEOUT : TSE_STATUS_OK;
+        s->error = failed ? TSE_STATUS_BARRIER_TIMEOUT : TSE_STATUS_OK;
         s->n_events = nev < 8 ? nev : 8;
         s->cycles = 0;
     }

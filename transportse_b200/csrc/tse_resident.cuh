@@ -21,7 +21,10 @@
 // values of the other colour, which they write after reading c.
 //
 // Every wait is bounded: a poll that runs out of time raises the launch's
-// error flag, which ends every other poll.
+// error flag, which ends every other poll.  A block whose wait ran out leaves
+// without storing its part of the result while its neighbours may go on to a
+// good end, so the last block to leave says whether the solve is good
+// (res_last).
 #pragma once
 
 #include "tse_common.cuh"
@@ -472,11 +475,26 @@ __device__ __forceinline__ bool res_team_sum(double& va, double& vb, ResSumShare
     return ok;
 }
 
-// A launch's exchange memory: a counter, the sum slots, and per colour one
+// The end of a launch's solve: every block comes here last, with `failed` if a
+// wait of its own ran out.  True in one thread of the launch, thread 0 of the
+// last block to come, with `failed` then if any block's did: it writes the
+// status.  No wait: the blocks count themselves.  (A barrier there slowed the
+// solves' loops by 1 %, by the registers' allocation.)
+template <int MODE>
+__device__ __forceinline__ bool res_last(unsigned* counter, unsigned nb, unsigned b, bool& failed) {
+    if (threadIdx.x != 0) return false;
+    if (MODE == RES_CLUSTER || nb == 1) return b == 0;
+    const unsigned before = atomicAdd(counter, failed ? 0x10001u : 1u);
+    failed = failed || (before >> 16) != 0u;
+    return (before & 0xffffu) == nb - 1u;
+}
+
+// A launch's exchange memory: two counters, the sum slots, and per colour one
 // record a group.
 constexpr size_t kResSlotBytes = (size_t)2 * kResSetWords * sizeof(uint64_t);
 struct ResMem {
     unsigned* counter;   // count_sync's
+    unsigned* leavers;   // res_last's
     uint64_t* slots;
     uint64_t* recs[2];
     int plane;
@@ -489,6 +507,7 @@ inline ResMem res_mem(void* at, const Layout& L, int vals) {
     const size_t groups = (size_t)L.nx * L.ny * ((L.H + vals - 1) / vals);
     ResMem m;
     m.counter = (unsigned*)at;
+    m.leavers = m.counter + 32;
     m.slots = (uint64_t*)((char*)at + 256);
     m.recs[0] = (uint64_t*)((char*)at + 256 + kResSlotBytes);
     m.recs[1] = m.recs[0] + 4 * groups;

@@ -45,10 +45,15 @@ __global__ void __launch_bounds__(128) selftest_wait_kernel(int which, GridBarri
 }
 
 // The resident solves' waits: an edge record and a sum record nobody writes
-// (result[0], result[1]: gave up, flags raised).
+// (result[0], result[1]: gave up, flags raised), and a solve that one block
+// leaves early.  There block 1's edge wait runs out; it still makes its partial
+// sum and leaves.  Block 0, late, finds that sum and knows of nothing
+// (result[2]: its sum is good); the last block to leave does (result[3]).
 __global__ void __launch_bounds__(kResMaxThreads) selftest_resident_kernel(int which, GridBarrier* bar,
-                                                                           uint64_t* words, int* result,
+                                                                           unsigned* counter, uint64_t* words,
+                                                                           int* result,
                                                                            unsigned long long timeout_ns) {
+    __shared__ ResSumShared sum;
     __shared__ uint4 ring[1];
     __shared__ int hrec[1], s_err;
     __shared__ unsigned short hp[1];
@@ -64,10 +69,26 @@ __global__ void __launch_bounds__(kResMaxThreads) selftest_resident_kernel(int w
         res_poll<kResMaxThreads>(words, 2, 1u, ring, hrec, hp, 1, bar, err, timeout_ns);
         __syncthreads();
         if (threadIdx.x == 0) result[0] = *err && *(volatile int*)&bar->error;
-    } else if (threadIdx.x == 0) {
-        double A = 0.0, B = 0.0;
-        const bool ok = res_poll_pair(slots, 1u, A, B, bar, err, timeout_ns);
-        result[1] = !ok && *err && *(volatile int*)&bar->error;
+    } else if (which == 1) {
+        if (threadIdx.x == 0) {
+            double A = 0.0, B = 0.0;
+            const bool ok = res_poll_pair(slots, 1u, A, B, bar, err, timeout_ns);
+            result[1] = !ok && *err && *(volatile int*)&bar->error;
+        }
+    } else {
+        const unsigned b = blockIdx.x;
+        if (b == 1) {
+            res_poll<kResMaxThreads>(words, 2, 1u, ring, hrec, hp, 1, bar, err, timeout_ns);
+        } else if (threadIdx.x == 0) {
+            const uint64_t t0 = globaltimer();
+            while (globaltimer() - t0 < 2 * timeout_ns) __nanosleep(1000);
+        }
+        __syncthreads();
+        double u = 1.0, v = 1.0;
+        const bool ok = res_team_sum<kResMaxThreads, RES_GRID>(u, v, sum, slots, 2u, b, 0u, bar, err, timeout_ns);
+        if (b == 0 && threadIdx.x == 0) result[2] = ok && u == 2.0 * kResMaxThreads;
+        bool failed = !ok;
+        if (res_last<RES_GRID>(counter, 2u, b, failed)) result[3] = failed;
     }
 }
 
@@ -121,15 +142,16 @@ extern "C" int32_t tse_selftest_resident_waits(int32_t* d_result, double timeout
     unsigned* counter = (unsigned*)((char*)d_ws + 256);
     uint64_t* w = (uint64_t*)((char*)d_ws + 512);
     int* result = (int*)d_result;
-    if (cudaMemsetAsync(d_result, 0, 3 * sizeof(int32_t), stream) != cudaSuccess) return TSE_ERR_LAUNCH;
-    for (int which = 0; which < 3; ++which) {
+    if (cudaMemsetAsync(d_result, 0, 5 * sizeof(int32_t), stream) != cudaSuccess) return TSE_ERR_LAUNCH;
+    for (int which = 0; which < 4; ++which) {
         if (cudaMemsetAsync(d_ws, 0, need, stream) != cudaSuccess) return TSE_ERR_LAUNCH;
-        if (which == 2) {
-            selftest_report_kernel<<<1, 1, 0, stream>>>(bar, counter, result + 2, ns);
+        if (which == 3) {
+            selftest_report_kernel<<<1, 1, 0, stream>>>(bar, counter, result + 4, ns);
             continue;
         }
-        void* args[] = {(void*)&which, (void*)&bar, (void*)&w, (void*)&result, (void*)&ns};
-        if (cudaLaunchCooperativeKernel((const void*)selftest_resident_kernel, dim3(1), dim3(kResMaxThreads), args, 0, stream) != cudaSuccess)
+        void* args[] = {(void*)&which, (void*)&bar, (void*)&counter, (void*)&w, (void*)&result, (void*)&ns};
+        if (cudaLaunchCooperativeKernel((const void*)selftest_resident_kernel, dim3(which == 2 ? 2 : 1),
+                                        dim3(kResMaxThreads), args, 0, stream) != cudaSuccess)
             return TSE_ERR_LAUNCH;
     }
     return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
