@@ -445,10 +445,12 @@ __global__ void __launch_bounds__(DcLayout<PIPES, WIDE>::kThreads, DcLayout<PIPE
     // the corrections were written by the kernel before (generic stores)
     if (producer) fence_proxy_async();
 
+    bool met = false;   // a barrier ended the last iteration
     for (int inner = 0; inner < c.cycle; ++inner) {
         num_it += 1;
         num_sub_it += 1;
         const bool check = c.pressure_schedule ? (num_it < 50 || num_it % 10 == 0) : true;
+        met = check;
         if (check) checkno += 1;
         float d2 = 0.0f, dd = 0.0f;
         for (int col = 0; col < 2; ++col, ++phases) {
@@ -623,6 +625,9 @@ __global__ void __launch_bounds__(DcLayout<PIPES, WIDE>::kThreads, DcLayout<PIPE
         const unsigned first = issued > (unsigned)ring ? issued - ring : 0u;
         for (unsigned v = first; v < issued; ++v) mbar_wait_bounded(&full[ring0 + v % ring], (v / ring) & 1u);
     }
+    // no block waits for another's last two phases: a block that gave up there
+    // is known to the leader only if all of them meet once more
+    if (event != EV_ERROR && !met && !count_sync(bar_count, ++bars * nb, c.bar)) event = EV_ERROR;
     if (leader) {
         st->t = t;
         st->dt = dt;
