@@ -187,8 +187,8 @@ def test_reports_and_gates_order_the_phases(pipes, groups):
 @pytest.mark.parametrize("pipes,groups", FORMS)
 def test_a_block_that_gave_up_is_known_at_the_end(pipes, groups):
     """The leader (block 0) may finish all its phases though another block gave
-    up in the last ones: its own flag does not tell, the blocks' last meeting
-    (a barrier that a block which gave up never reaches) does."""
+    up in the last ones: its own flag does not tell, the blocks' marks as they
+    leave do."""
     rng = random.Random(pipes + groups)
     own_flag_passes = 0
     for n in range(60):

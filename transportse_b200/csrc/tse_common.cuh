@@ -156,6 +156,15 @@ __device__ __forceinline__ bool count_sync(unsigned* counter, unsigned target, G
     return s_ok != 0;
 }
 
+// A launch's blocks count themselves out, each once, by one thread, with
+// `failed` if a wait of the block ran out: true for the last one, with `failed`
+// then if any block's did.  No block waits.
+__device__ __forceinline__ bool last_out(unsigned* counter, unsigned nblocks, bool& failed) {
+    const unsigned before = atomicAdd(counter, failed ? 0x10001u : 1u);
+    failed = failed || (before >> 16) != 0u;
+    return (before & 0xffffu) == nblocks - 1u;
+}
+
 // ---------------------------------------------------------- block reduces
 template <int NT>
 __device__ __forceinline__ double block_sum(double v, double* sh) {

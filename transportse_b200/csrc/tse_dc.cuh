@@ -328,9 +328,10 @@ inline void sweep_head(const Layout& L, long long nb, TmaStage& T) {
     T.first = T.head + (int)far;
 }
 constexpr int kSegs = 2;
-// words from the barrier counter to report s's counter (a sector each)
+// words from the barrier counter to report s's counter (a sector each), and to
+// the counter of the blocks that have left
 constexpr int kSegWords = 8, kSegBase = 32;
-constexpr size_t kProgBytes = (kSegBase + kSegs * kSegWords) * sizeof(unsigned);
+constexpr size_t kProgBytes = (kSegBase + (kSegs + 1) * kSegWords) * sizeof(unsigned);
 
 // a report's count has reached `target` (acquire); bounded
 __device__ __forceinline__ bool seg_wait(const unsigned* count, unsigned target, GridBarrier* bar, volatile int* err,

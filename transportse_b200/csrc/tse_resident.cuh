@@ -484,9 +484,7 @@ template <int MODE>
 __device__ __forceinline__ bool res_last(unsigned* counter, unsigned nb, unsigned b, bool& failed) {
     if (threadIdx.x != 0) return false;
     if (MODE == RES_CLUSTER || nb == 1) return b == 0;
-    const unsigned before = atomicAdd(counter, failed ? 0x10001u : 1u);
-    failed = failed || (before >> 16) != 0u;
-    return (before & 0xffffu) == nb - 1u;
+    return last_out(counter, nb, failed);
 }
 
 // A launch's exchange memory: two counters, the sum slots, and per colour one
