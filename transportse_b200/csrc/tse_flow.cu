@@ -467,15 +467,16 @@ __global__ void l2_partial_kernel(const double* New, const double* Old, long lon
 // dt_CFL (tse.py:1241-1246): element f of reshape(|qx|/phi, (ny,nz,nx)) / dx
 // is divided by dx[f % nx]; likewise dy[f % ny]; qz uses dz[k].
 // Bound: DRAM.  |q| / p / d is formed only where it can exceed the warp's
-// maximum so far (a product tells, with a margin for its rounding; anything
-// near an end of the exponent range, and NaN, is formed): of 160 us at
+// maximum so far.  A product tells, with a margin for its rounding, where the
+// maximum, p and d are positive and far from the ends of the exponent range
+// (|q| / p may then round to nothing without reaching the maximum); with any
+// other, and with NaN, the quotient is formed.  Of 160 us at
 // 255 x 256 x 127 the arrays take 41; six divisions and two 64-bit remainders a
 // cell took the rest.  Now 86.
 struct CflMax {
     double m = -HUGE_VAL;   // the warp's
     __device__ __forceinline__ bool below(double q, double p, double d) const {
-        const double mp = m * p, t = mp * d;
-        return mp < 1e290 && t > 1e-290 && t < 1e290 && q * (1.0 + 1e-12) < t;
+        return plain_positive(m) && plain_positive(p) && plain_positive(d) && q * (1.0 + 1e-12) < m * p * d;
     }
     __device__ __forceinline__ void take(double q, double p, double d, bool in) {
         const bool cand = in && !below(q, p, d);
