@@ -10,6 +10,7 @@
 //                        + (1-omega) (...) + R Xn + W - E) / (R - omega M)
 // (tse.py:870-875, 1038-1043) term by term.  Compiled with --fmad=false.
 #include <algorithm>
+#include <cmath>
 
 #include "tse_dc.cuh"
 #include "tse_forms.cuh"
@@ -458,6 +459,12 @@ __device__ __forceinline__ double qdiv(double a, double2 b) {
     const double r = __fma_rn(__fma_rn(-b.x, q, a), b.y, q);
     return (__double2hiint(q) & 0x7ff00000) == 0x7ff00000 ? q : r;   // inf, NaN
 }
+// A divisor and its reciprocal.  An infinite one (a steady state's dt, a product
+// of spacings) goes along as {0, 0}: the correction is then 0, where -inf 0 + a
+// would be NaN, and the quotient a 0.
+__device__ __forceinline__ double2 with_reciprocal(double b) {
+    return fabs(b) < HUGE_VAL ? make_double2(b, 1.0 / b) : make_double2(b == b ? 0.0 : b, b == b ? 0.0 : b);
+}
 // |v| far from both ends of the exponent range (and not 0, inf or NaN)
 __device__ __forceinline__ bool mid_range(double v) {
     const unsigned e = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu;
@@ -492,7 +499,9 @@ __global__ void axis_tables_kernel(TseGrid g, double2* tab) {
         b[3] = d[i + 1] + dd;
     }
     if (i > 0) b[2] = (0.5 * (d[i - 1] + dd)) * dd;
-    for (int q = 0; q < kTabPairs; ++q) t[q * st] = make_double2(b[q], 1.0 / b[q]);
+    // the first and the last divisor are spacings too
+    for (int q = 0; q < kTabPairs; ++q)
+        t[q * st] = q == 1 || q == 2 ? with_reciprocal(b[q]) : make_double2(b[q], 1.0 / b[q]);
 }
 static size_t axis_table_bytes(const Layout& L) {
     return align256((size_t)(L.nx + L.ny + L.nz) * kTabPairs * sizeof(double2));
@@ -626,7 +635,7 @@ __global__ void __launch_bounds__(kBlock, Kind::kBlocks)
     assemble_fast_kernel(TseGrid g, typename Kind::Args a, TransportForm F, uint8_t* mask0, uint8_t* mask1,
                          Layout L, const double2* __restrict__ tab, DcFuse fz) {
     __shared__ double sh[kBlock / 32];
-    const double2 dt = make_double2(a.dt, 1.0 / a.dt);
+    const double2 dt = with_reciprocal(a.dt);
     const double omega = F.omega;
     const long long N = F.Ncal;
     const int ts = L.nx + L.ny + L.nz;
