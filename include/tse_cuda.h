@@ -434,6 +434,11 @@ int32_t tse_selftest_bounded_waits(int32_t *d_result, double timeout_s, void *d_
 int32_t tse_selftest_resident_waits(int32_t *d_result, double timeout_s, void *d_ws,
                                     size_t ws_bytes, void *stream);
 
+/* The flux kernels' quotients q = a / b (b positive) and reciprocals y = 1 / b of
+ * n pairs of device values, as they form them. */
+int32_t tse_selftest_quotients(const double *a, const double *b, double *q, double *y, int64_t n,
+                               void *stream);
+
 /* Batched solves run so far by the fused form's device-driven loop and by its
  * host loop (TseDcOptions.host_loop; no counterpart in the reference). */
 int32_t tse_batch_loop_stats(int64_t *graph_solves, int64_t *host_solves);

@@ -139,6 +139,7 @@ SIGNATURES = {
                              _P]),
     "tse_selftest_bounded_waits": (_I, [_P, _D, _P, _S, _P]),
     "tse_selftest_resident_waits": (_I, [_P, _D, _P, _S, _P]),
+    "tse_selftest_quotients": (_I, [_P, _P, _P, _P, ct.c_int64, _P]),
     "tse_batch_loop_stats": (_I, [ct.POINTER(ct.c_int64), ct.POINTER(ct.c_int64)]),
     "tse_version": (ct.c_char_p, []),
 }

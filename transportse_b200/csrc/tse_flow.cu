@@ -5,6 +5,7 @@
 #include <cmath>
 
 #include "tse_common.cuh"
+#include "tse_quotient.cuh"
 
 namespace tse {
 
@@ -14,50 +15,6 @@ __device__ __forceinline__ void decode(long long t, int ny, int nz, int& i, int&
     long long row;
     grid_coords(t, ny, nz, i, j, k, row);
 }
-
-// ------------------------------------------------------ exact quotients
-// FP64 divisions bound the two flux kernels, 26 a cell in compute_q and 25 in
-// flow_error by the formulas: an operator's branch for special operands keeps
-// one from overlapping the next, and each does its own reciprocal.  Here a
-// reciprocal is formed once a divisor and correctly rounded, and quotients by
-// it take two fused corrections (Markstein 1990, "Computation of elementary
-// functions on the IBM RISC System/6000": from a faithful y,
-// y + (1 - b y) y = RN(1 / b) unless b's significand is all ones, and from a
-// faithful q and that y, q + (a - b q) y = RN(a / b)), without a branch.  The
-// results are the divided quotients' bits as long as no operand is near an end
-// of the exponent range; a cell that has another operand is formed by the
-// formulas' own divisions (*_cell).
-struct Divisor {
-    double b, y;
-};
-__device__ __forceinline__ Divisor divisor(double b) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));   // to 2^-20
-    const double e = __fma_rn(-b, y, 1.0);
-    y = __fma_rn(y, __fma_rn(e, e, e), y);
-    return {b, __fma_rn(__fma_rn(-b, y, 1.0), y, y)};
-}
-__device__ __forceinline__ double quotient(double a, const Divisor& d) {
-    double q = a * d.y;
-    q = __fma_rn(__fma_rn(-d.b, q, a), d.y, q);
-    return __fma_rn(__fma_rn(-d.b, q, a), d.y, q);
-}
-// a may be zero: keeps its sign
-__device__ __forceinline__ double quotient_0(double a, const Divisor& d) {
-    return a == 0.0 ? a * d.y : quotient(a, d);
-}
-__device__ __forceinline__ Divisor half(const Divisor& s) { return {0.5 * s.b, 2.0 * s.y}; }
-// positive, within 2^-80 .. 2^80: what the formulas derive from such inputs
-// stays within 2^-900 .. 2^900
-__device__ __forceinline__ bool plain_positive(double v) {
-    return (unsigned)__double2hiint(v) - (943u << 20) <= (160u << 20);
-}
-// 0 or of magnitude 2^-300 .. 2^300
-__device__ __forceinline__ bool plain_signed(double v) {
-    return v == 0.0 || ((unsigned)__double2hiint(v) & 0x7fffffffu) - (723u << 20) <= (600u << 20);
-}
-__device__ __forceinline__ bool not_all_ones(double b) { return __double2loint(b) != -1; }
-__device__ __forceinline__ bool plain_divisor(double b) { return plain_positive(b) && not_all_ones(b); }
 
 // The flux kernels walk along x with a warp on 32 consecutive cells of the
 // (y, z) plane: the x face and its quotients stay in registers, a z face's come
@@ -69,7 +26,7 @@ constexpr int kWalkMax = 16;
 // thread a cell against walks: fluxes 31 / 33 at 96^3, 56 / 51 at 112^3, 130 / 105
 // at 160 x 192 x 101; flow error 5.2 / 6.5 at 48^3, 16 / 14 at 80^3, 99 / 75).
 constexpr long long kWalkCellsQ = 1200000, kWalkCellsE = 400000;
-constexpr int kWalkBlocksQ = 4, kWalkBlocksE = 3;   // resident on a SM
+constexpr int kWalkBlocksQ = 4, kWalkBlocksE = 4;   // resident on a SM
 constexpr int kWalkWarps = kBlock / 32;
 struct Walk {
     int steps;                // cells of a walk
@@ -105,12 +62,12 @@ struct WalkX {
             const int i = i0 - 1 + q;
             const double a = i >= 0 && i < g.nx ? g.dx[i] : 1.0;
             d[q] = a;
-            ok = ok && plain_divisor(a);
+            ok = ok && plain_positive(a);
             if (q < kWalkMax + 1) {
                 const double b = i + 1 < g.nx ? g.dx[i + 1] : 1.0;
                 own[q] = divisor(a);
                 sum[q] = divisor(b + a);
-                ok = ok && plain_divisor(b + a);
+                ok = ok && plain_positive(b + a);
             }
         }
         return __syncthreads_and(ok);
@@ -176,15 +133,13 @@ struct Perm {
 __device__ __forceinline__ Perm perm(double K, double d, bool& ok) {
     const bool z = K == 0.0;
     const double s = z ? 1.0 : K;
-    ok = ok && plain_divisor(s);
+    ok = ok && plain_positive(s);
     return {quotient(d, divisor(s)), z};
 }
 // -harm2(K) / harm2(nue) of a face
-__device__ __forceinline__ double mobility(double dsum, const Perm& a, const Perm& b, double n1, double n2,
-                                           bool& ok) {
+__device__ __forceinline__ double mobility(double dsum, const Perm& a, const Perm& b, double n1, double n2) {
     const double sk = a.a + b.a, sn = n1 + n2;
     const double hk = quotient(dsum, divisor(sk)), hn = quotient(dsum, divisor(sn));
-    ok = ok && not_all_ones(sk) && not_all_ones(sn) && not_all_ones(hn);
     return quotient_0(a.zero || b.zero ? -0.0 : -hk, divisor(hn));
 }
 
@@ -211,10 +166,10 @@ __global__ void __launch_bounds__(kBlock, kWalkBlocksQ)
     const double dy0 = g.dy[j], dy1 = hy ? g.dy[j + 1] : 1.0, dz0 = g.dz[k], dz1 = hz ? g.dz[k + 1] : 1.0;
     const Divisor sy = divisor(dy1 + dy0), sz = divisor(dz1 + dz0);
     okd = okd && plain_positive(dy0) && plain_positive(dy1) && plain_positive(dz0) && plain_positive(dz1) &&
-          plain_divisor(sy.b) && plain_divisor(sz.b);
+          plain_positive(sy.b) && plain_positive(sz.b);
     long long t = (long long)i0 * plane + c0;
     double p = P[t], r = rho[t], n = nue[t], bp = BP[t];
-    bool ok0 = okd && plain_divisor(n) && plain_positive(r);   // the cell's own values
+    bool ok0 = okd && plain_positive(n) && plain_positive(r);   // the cell's own values
     Divisor nd = divisor(n);
     Perm ax = perm(Kx[t], X.d[1], ok0);
     double an = quotient(X.d[1], nd);
@@ -227,10 +182,10 @@ __global__ void __launch_bounds__(kBlock, kWalkBlocksQ)
         const double ky = Ky[t], kz = Kz[t], kyo = Ky[ty], no = nue[ty], po = P[ty], bo = BP[ty];
         const double pz = P[tz], rz = rho[tz], bz = BP[tz];
         const Divisor nd1 = divisor(n1);
-        bool ok1 = okd && plain_divisor(n1) && plain_positive(r1);
+        bool ok1 = okd && plain_positive(n1) && plain_positive(r1);
         const Perm ax1 = perm(kx1, X.d[s + 2], ok1);
         const double an1 = quotient(X.d[s + 2], nd1);
-        bool ok = ok0 && ok1 && plain_divisor(no) && plain_positive(rz);
+        bool ok = ok0 && ok1 && plain_positive(no) && plain_positive(rz);
         Perm zk = perm(kz, dz0, ok);
         const double zn = quotient(dz0, nd);
         const unsigned good = __ballot_sync(0xffffffffu, ok), zero = __ballot_sync(0xffffffffu, zk.zero);
@@ -240,12 +195,12 @@ __global__ void __launch_bounds__(kBlock, kWalkBlocksQ)
         const double px = p1 - p, py = po - p, pu = pz - p;
         ok = ok && plain_signed(px) && plain_signed(py) && plain_signed(pu);
         const Divisor sx = X.sum[s + 1];
-        const double vx = mobility(sx.b, ax1, ax, an1, an, ok) *
+        const double vx = mobility(sx.b, ax1, ax, an1, an) *
                           (quotient_0(px, half(sx)) + quotient(r1 * X.d[s + 2] + r * X.d[s + 1], sx) * g.g * g.sin_beta);
         const double vy = quotient_0(mobility(sy.b, perm(kyo, dy1, ok), perm(ky, dy0, ok), quotient(dy1, divisor(no)),
-                                              quotient(dy0, nd), ok) * py,
+                                              quotient(dy0, nd)) * py,
                                      half(sy));
-        const double vz = mobility(sz.b, zk1, zk, zn1, zn, ok) *
+        const double vz = mobility(sz.b, zk1, zk, zn1, zn) *
                           (quotient_0(pu, half(sz)) + quotient(rz * dz1 + r * dz0, sz) * g.g * g.cos_beta);
         if (out) {
             if (ok) {
@@ -307,8 +262,7 @@ __global__ void flow_error_cells_kernel(TseGrid g, const double* P, const double
 }
 
 // harm2 from its two quotients
-__device__ __forceinline__ double harm_of(double dsum, double a1, double a2, bool& ok) {
-    ok = ok && not_all_ones(a1 + a2);
+__device__ __forceinline__ double harm_of(double dsum, double a1, double a2) {
     return quotient(dsum, divisor(a1 + a2));
 }
 
@@ -335,18 +289,18 @@ __global__ void __launch_bounds__(kBlock, kWalkBlocksE)
     const double dy1 = hy ? g.dy[j + 1] : 1.0, dy2 = ly ? g.dy[j - 1] : 1.0;
     const double dz1 = hz ? g.dz[k + 1] : 1.0;
     const Divisor dy = divisor(g.dy[j]), dz = divisor(g.dz[k]), dt = divisor(dt_P);
-    okd = okd && plain_divisor(dy.b) && plain_divisor(dz.b) && plain_divisor(dt_P) && plain_positive(dy1) &&
+    okd = okd && plain_positive(dy.b) && plain_positive(dz.b) && plain_positive(dt_P) && plain_positive(dy1) &&
           plain_positive(dy2) && plain_positive(dz1);
     long long t = (long long)i0 * plane + c0;
     double r = rho[t];
-    bool ok0 = okd && plain_divisor(r), okm = true;   // this cell's density; the face before
+    bool ok0 = okd && plain_positive(r), okm = true;   // this cell's density; the face before
     Divisor rd = divisor(r);
     double ar = quotient(X.d[1], rd), q0 = 0.0, fx = 0.0;
     if (i0 != 0) {
         const double rm = rho[t - plane];
         q0 = qx[t - plane];
-        okm = ok0 && plain_divisor(rm) && plain_signed(q0);
-        fx = harm_of(X.d[0] + X.d[1], quotient(X.d[0], divisor(rm)), ar, okm);
+        okm = ok0 && plain_positive(rm) && plain_signed(q0);
+        fx = harm_of(X.d[0] + X.d[1], quotient(X.d[0], divisor(rm)), ar);
     }
     const int steps = min(w.steps, nx - i0);
     for (int s = 0; s < steps; ++s, t += plane) {
@@ -359,23 +313,23 @@ __global__ void __launch_bounds__(kBlock, kWalkBlocksE)
         const double zr = quotient(dz.b, rd);
         bool ok = ok0;
         const double zr1 = __shfl_down_sync(0xffffffffu, zr, 1);
-        const double fz = harm_of(dz1 + dz.b, zr1, zr, ok);
+        const double fz = harm_of(dz1 + dz.b, zr1, zr);
         const double fz0 = __shfl_up_sync(0xffffffffu, fz, 1);
         // the lanes beside: their densities (and the face of the one before)
         const unsigned good = __ballot_sync(0xffffffffu, ok);
         ok = ok && (!hz || (good >> ((lane + 1) & 31) & 1u)) && (!lz || (good >> ((lane + 31) & 31) & 1u));
         // the next x face
         const Divisor rd1 = divisor(r1);
-        const bool ok1 = okd && plain_divisor(r1);
+        const bool ok1 = okd && plain_positive(r1);
         const double ar1 = quotient(X.d[s + 2], rd1);
         bool okx = ok0 && ok1 && plain_signed(q0);
-        fx = harm_of(X.sum[s + 1].b, ar1, ar, okx);
-        ok = ok && okx && okm && plain_divisor(ra) && plain_divisor(rb) && plain_signed(qa) && plain_signed(qb) &&
+        fx = harm_of(X.sum[s + 1].b, ar1, ar);
+        ok = ok && okx && okm && plain_positive(ra) && plain_positive(rb) && plain_signed(qa) && plain_signed(qb) &&
              plain_signed(qu) && plain_signed(qd);
         const Divisor dx = X.own[s + 1];
         const double yr = quotient(dy.b, rd);
-        const double fa = harm_of(dy1 + dy.b, quotient(dy1, divisor(ra)), yr, ok);
-        const double fb = harm_of(dy2 + dy.b, quotient(dy2, divisor(rb)), yr, ok);
+        const double fa = harm_of(dy1 + dy.b, quotient(dy1, divisor(ra)), yr);
+        const double fb = harm_of(dy2 + dy.b, quotient(dy2, divisor(rb)), yr);
         double v = 0.0;
         if (hx) v -= (quotient_0(q0, dx) * fx);
         if (lx) v += (quotient_0(qm, dx) * fm);

@@ -9,6 +9,7 @@
 // instead of holding the GPU.  Nothing faults: the kernels only wait, give up
 // and return.
 #include "tse_dc.cuh"
+#include "tse_quotient.cuh"
 #include "tse_resident.cuh"
 
 namespace tse {
@@ -101,6 +102,15 @@ __global__ void selftest_report_kernel(GridBarrier* bar, unsigned* counter, int*
     *result = !ok && s_err && *(volatile int*)&bar->error;
 }
 
+// The flux kernels' quotients and reciprocals, for a comparison with divisions
+__global__ void selftest_quotient_kernel(const double* a, const double* b, double* q, double* y, long long n) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const Divisor d = divisor(b[t]);
+    q[t] = quotient_0(a[t], d);
+    y[t] = d.y;
+}
+
 }  // namespace tse
 
 using namespace tse;
@@ -154,5 +164,13 @@ extern "C" int32_t tse_selftest_resident_waits(int32_t* d_result, double timeout
                                         dim3(kResMaxThreads), args, 0, stream) != cudaSuccess)
             return TSE_ERR_LAUNCH;
     }
+    return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
+}
+
+extern "C" int32_t tse_selftest_quotients(const double* a, const double* b, double* q, double* y, int64_t n,
+                                          void* stream_) {
+    if (!a || !b || !q || !y || n < 1 || n > (1LL << 31)) return TSE_ERR_ARG;
+    selftest_quotient_kernel<<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, 0, (cudaStream_t)stream_>>>(a, b, q, y,
+                                                                                                       n);
     return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
 }
