@@ -73,8 +73,9 @@ typedef struct TseSolveStatus {
     double ev_dt[8];
     double ev_diff[8];
     int32_t cycles;    /* mixed-precision forms: FP64 residual evaluations */
-    int32_t reserved;
+    int32_t sweep;     /* FP64 forms: the kernel that ran, TSE_SWEEP_*; else 0 */
 } TseSolveStatus;
+enum { TSE_SWEEP_PLAIN = 1, TSE_SWEEP_STAGED = 2, TSE_SWEEP_RESIDENT = 3 };
 
 /* Pressure solve arguments, compute_P(P, c_f, nue, rho_f, phi, Kx, Ky, Kz,
  * qx, qy, qz, dt_P, BP, WP, SOR, max_it, inc_it, max_dt, min_dt, P_conv)

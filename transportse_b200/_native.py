@@ -18,6 +18,11 @@ TSE_WS_REDUCE = 3
 TSE_WS_PRESSURE_DC = 4
 TSE_WS_TRANSPORT_DC = 5
 
+# the FP64 kernel that ran (TseSolveStatus.sweep)
+TSE_SWEEP_PLAIN = 1
+TSE_SWEEP_STAGED = 2
+TSE_SWEEP_RESIDENT = 3
+
 ERRORS = {-1: "invalid argument", -2: "workspace too small", -3: "kernel launch failed",
           -4: "device error"}
 
@@ -36,7 +41,7 @@ class TseSolveStatus(ct.Structure):
                 ("converged", ct.c_int32), ("num_it", ct.c_int32), ("num_sub_it", ct.c_int32),
                 ("halvings", ct.c_int32), ("error", ct.c_int32), ("n_events", ct.c_int32),
                 ("ev_it", ct.c_int32 * 8), ("ev_dt", ct.c_double * 8),
-                ("ev_diff", ct.c_double * 8), ("cycles", ct.c_int32), ("reserved", ct.c_int32)]
+                ("ev_diff", ct.c_double * 8), ("cycles", ct.c_int32), ("sweep", ct.c_int32)]
 
 
 def _ptr_fields(names):

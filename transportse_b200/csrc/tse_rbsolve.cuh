@@ -174,6 +174,7 @@ __global__ void __launch_bounds__(kPlainBlock, 1) rb_solve_kernel(Form F, SolveC
         s->error = err ? TSE_STATUS_BARRIER_TIMEOUT : TSE_STATUS_OK;
         s->n_events = nev < 8 ? nev : 8;
         s->cycles = 0;
+        s->sweep = TSE_SWEEP_PLAIN;
     }
 }
 

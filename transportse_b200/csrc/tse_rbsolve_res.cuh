@@ -283,6 +283,7 @@ __global__ void __launch_bounds__(kXResThreads, 1)
         s->error = failed ? TSE_STATUS_BARRIER_TIMEOUT : TSE_STATUS_OK;
         s->n_events = nev < 8 ? nev : 8;
         s->cycles = 0;
+        s->sweep = TSE_SWEEP_RESIDENT;
     }
 }
 

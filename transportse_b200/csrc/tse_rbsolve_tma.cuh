@@ -365,6 +365,7 @@ __global__ void __launch_bounds__(kXThreads, TSE_X_MINB) rb_solve_tma_kernel(For
         s->error = fail ? TSE_STATUS_BARRIER_TIMEOUT : TSE_STATUS_OK;
         s->n_events = nev < 8 ? nev : 8;
         s->cycles = 0;
+        s->sweep = TSE_SWEEP_STAGED;
     }
 }
 

@@ -75,8 +75,10 @@ class Model:
         self.last_status = None
         self.launches = 0
         # FP64 solves' sweep kernel (args.sweep): 0 resident where the grid
-        # fits on the chip, else staged; 1 plain loads; 2 the bulk-copy staged
-        # kernel where its stages fit; same cell values
+        # fits on the chip, else plain loads below a million cells of a colour,
+        # else as 2; 1 plain loads; 2 the bulk-copy staged kernel where its
+        # stages fit, else plain.  Same cell values; last_status.sweep says
+        # which one ran
         self.sweep = 0
         # mixed-precision solves: the staged FP32 sweep's variant (chunk
         # cells, ring stages, pipelines per block; 0 = the library's
