@@ -11,9 +11,9 @@ from transportse_b200._native import TSE_SWEEP_STAGED as STAGED
 pytestmark = pytest.mark.gpu
 
 # shape; the kernels of a pressure solve with sweep 0 and 2 (1 is plain) and of a species
-# solve.  (3, 2, 1000): rings of two stages; (1, 2, 3000): the pressure solve's stages fit no
-# ring; 184,320 cells of a colour, the resident range's bound, and a grid too large for its
-# shared memory below that; a million cells of a colour, where staged begins
+# solve.  (3, 2, 1000): rings of two stages; (1, 2, 3000): a column too long for a
+# block's shared memory, and the pressure solve's stages fit no ring; grids whose state does
+# not fit the SMs' shared memory; either side of a million cells of a colour
 CASES = [((64, 48, 40), (RESIDENT, STAGED), (RESIDENT, STAGED)),
          ((37, 23, 51), (RESIDENT, STAGED), (RESIDENT, STAGED)),
          ((3, 2, 1000), (RESIDENT, STAGED), (RESIDENT, STAGED)),
