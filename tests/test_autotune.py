@@ -1,0 +1,60 @@
+"""The autotuners' choices, with the timings made up."""
+import types
+
+import pytest
+
+from transportse_b200 import autotune
+
+
+class _Field:
+    def clone(self):
+        return self
+
+    def copy_(self, other):
+        return self
+
+
+def _sim(max_blocks=0, index=0, shape=(40, 40, 40)):
+    M = types.SimpleNamespace(precision="fp32dc", nx=shape[0], ny=shape[1], nz=shape[2], max_blocks=max_blocks,
+                              device=types.SimpleNamespace(index=index), sweep_variant=None)
+    return types.SimpleNamespace(M=M, S={"P": _Field()})
+
+
+@pytest.fixture
+def timings(monkeypatch):
+    """us(max_blocks, variant) -> (us an iteration, the variant that ran)"""
+    made = {}
+
+    def timed(sim, variant, iters):
+        us, ran = made["us"](sim.M.max_blocks, tuple(variant))
+        return 1e-3 * us * iters, iters, ran
+
+    monkeypatch.setattr(autotune, "_timed_solve", timed)
+    monkeypatch.setattr(autotune.torch.cuda, "synchronize", lambda: None)
+    monkeypatch.setattr(autotune, "_chosen", {})
+    return made
+
+
+def test_a_capped_models_choice_is_not_an_uncapped_ones(timings):
+    """Under a block cap the grid streams, without one it is resident: each
+    model gets its own choice, and so does another device's."""
+    def us(cap, v):
+        if any(v):
+            return (7.0 if v == (256, 4, 1) else 8.0), v
+        return (9.0, (512, 4, 2)) if cap else (2.0, (0, 0, 0))
+
+    timings["us"] = us
+    assert autotune.tune_sweep(_sim(max_blocks=8))["variant"] == (256, 4, 1)
+    free = _sim()
+    assert autotune.tune_sweep(free)["variant"] == (0, 0, 0) == free.M.sweep_variant
+    assert autotune.tune_sweep(_sim())["cached"]
+    assert "cached" not in autotune.tune_sweep(_sim(index=1))
+
+
+def test_the_librarys_choice_keeps_its_name(timings):
+    """Where asking for nothing wins, nothing is asked for later either, though
+    a staged variant ran."""
+    timings["us"] = lambda cap, v: (5.0, (512, 4, 2)) if not any(v) else (6.0, v)
+    rec = autotune.tune_sweep(_sim())
+    assert rec["variant"] == (0, 0, 0)
+    assert min(rec["trials"], key=lambda t: t["us_per_iteration"])["chunk"] == 512

@@ -16,8 +16,8 @@ single launch):
 ``tune_sweep`` times each variant on the model's own pressure solve (exactly
 ``iters`` red+black iterations, the sweep kernel's own event time, the state
 restored afterwards) and sets the fastest as the model's ``sweep_variant``;
-the choice is kept per grid shape, so later models of the same shape take it
-without timing.  The variant changes only how the same cell updates are
+the choice is kept per device, block cap and grid shape, so later models of the
+same take it without timing.  The variant changes only how the same cell updates are
 scheduled: every cell update is the same; only the grouping of the
 convergence check's sums follows the chunking, so the solves agree bit for bit
 unless a norm falls within rounding of its tolerance.  SOR's omega is not a knob
@@ -71,7 +71,9 @@ def tune_sweep(sim, iters=64, repeats=3, variants=VARIANTS, cache=True):
     M = sim.M
     if M.precision != "fp32dc":
         raise ValueError("the sweep autotuner is for the mixed-precision form")
-    key = (M.nx, M.ny, M.nz)
+    # whether the grid can be resident depends on the device and the block cap
+    index = M.device.index if M.device.index is not None else torch.cuda.current_device()
+    key = (index, getattr(M, "max_blocks", 0), M.nx, M.ny, M.nz)
     if cache and key in _chosen:
         M.sweep_variant = _chosen[key]["variant"]
         return dict(_chosen[key], cached=True)
@@ -94,7 +96,8 @@ def tune_sweep(sim, iters=64, repeats=3, variants=VARIANTS, cache=True):
         if ran is None or ran in seen or (ran[0] == 0 and any(v)):
             continue   # the plain-load sweep ran, or a variant already timed
         seen.add(ran)
-        trials.append({"chunk": ran[0], "ring": ran[1], "pipes": ran[2],
+        # (0, 0, 0) stays a choice of the library's, whatever ran under it
+        trials.append({"chunk": ran[0], "ring": ran[1], "pipes": ran[2], "asked": tuple(v),
                        "us_per_iteration": 1e3 * statistics.median(ms_list)})
     torch.cuda.synchronize()
     if not trials:
@@ -102,7 +105,7 @@ def tune_sweep(sim, iters=64, repeats=3, variants=VARIANTS, cache=True):
         return {"variant": (0, 0, 0), "trials": [], "failed": failed,
                 "note": "no variant ran"}
     best = min(trials, key=lambda t: t["us_per_iteration"])
-    rec = {"variant": (best["chunk"], best["ring"], best["pipes"]),
+    rec = {"variant": best["asked"] if not any(best["asked"]) else (best["chunk"], best["ring"], best["pipes"]),
            "us_per_iteration": best["us_per_iteration"], "iters": iters, "trials": trials}
     if failed:
         rec["failed"] = failed
