@@ -319,7 +319,9 @@ class Ensemble:
                             stream.synchronize()
                     except Exception as e:   # reported after all workers stop
                         errors.append((i, e))
-                        stream.synchronize()
+                        # a batched solve that failed may still run on the
+                        # gate's stream, on memory the next run is given
+                        torch.cuda.synchronize(self.device)
                     sims[i] = None   # its device memory goes back to the pool
 
             threads = [threading.Thread(target=stepper, args=(st,), daemon=True) for st in step_streams]
