@@ -73,7 +73,9 @@ class StreamShelf:
     five models spent half of its 240 ms in some 50 cudaMalloc calls, run
     after run.  A stream taken back is lent again for the same role (what a
     role allocates is alike), at most ``KEEP`` lying idle per device and role.
-    A stream is lent to one holder at a time."""
+    A stream object is lent to one holder at a time; PyTorch makes such objects
+    over a pool of 32 CUDA streams a device, so beyond that two of them may be
+    one stream, whose work then runs in order."""
     KEEP = 32
 
     def __init__(self):
