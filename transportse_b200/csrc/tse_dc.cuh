@@ -370,17 +370,17 @@ __host__ __device__ inline TmaStage tma_stage(int H, int C = kTmaChunk) {
     return t;
 }
 
-// A chunk of the colour being swept, in two parts: its record block and (where
-// the consumers do not read it themselves) its own old correction, which add
-// their bytes to the stage's transaction count without arriving, and the three
-// windows of the other colour, which carry the stage's single arrival.  The
-// block is copied whole; dw: cnt cells from the chunk's first, or null.
+// A chunk of the colour being swept, in two parts: its record block and its own
+// old correction, which add their bytes to the stage's transaction count without
+// arriving, and the three windows of the other colour, which carry the stage's
+// single arrival.  The block is copied whole; dw: cnt cells from the chunk's
+// first.
 __device__ __forceinline__ void tma_issue_own(const TmaStage& T, unsigned char* stage, uint64_t* bar,
                                               const float* block, const float* dw, long long cnt) {
-    const unsigned b_blk = (unsigned)(29 * T.chunk), b_dw = dw ? (unsigned)(4 * cnt) : 0u;
+    const unsigned b_blk = (unsigned)(29 * T.chunk), b_dw = (unsigned)(4 * cnt);
     mbar_add_tx(bar, b_blk + b_dw);
     bulk_g2s_hint(stage + T.rec, block, b_blk, bar, l2_evict_first());
-    if (dw) bulk_g2s_hint(stage + T.dw, dw, b_dw, bar, l2_evict_last());
+    bulk_g2s_hint(stage + T.dw, dw, b_dw, bar, l2_evict_last());
 }
 
 __device__ __forceinline__ void tma_issue_windows_n(long long SX, int H, const TmaStage& T,
@@ -404,16 +404,18 @@ __device__ __forceinline__ void tma_issue_windows(const DcCtl& c, const TmaStage
     tma_issue_windows_n(c.L.SX, c.L.H, T, stage, bar, dq, m0);
 }
 
-// Roles: warps 0-7 consume, in two groups of four warps; group g computes the
-// block's chunks i = g, g + 2, ..., so two chunks are in computation at once
-// and neither waits for the other.  Warp 8 produces: its lane 0 issues the
-// copies of chunk i into stage i % kTmaStages as soon as the consumers of
-// chunk i - kTmaStages have released that stage (`empty` barrier, one arrival
-// per consumer warp).  Consumers wait on the stage's `full` barrier (the
-// copies' byte count).  Only the colour phases end in block- and grid-wide
-// barriers.  Every wait is bounded; a wait that runs out raises a block flag
-// that ends every other wait of the block, and the kernel leaves with
-// EV_ERROR after the copies still in flight have landed (again bounded).
+// Roles of a staged sweep's block: consumer warps in groups of four, a chunk a
+// group at a time, so that two or more chunks are in computation at once and
+// none waits for another; producer warps, whose lane 0 issues a chunk's copies
+// into the next stage of its ring as soon as that stage's last chunk has been
+// released (`empty` barrier, one arrival per consumer warp).  Consumers wait on
+// the stage's `full` barrier (the copies' byte count).  The batched sweep has
+// a producer and a ring for each of its two groups, and its colour phases end in
+// block- and device-wide barriers; the single-model sweep's rings, groups and
+// phases are described at dc_sweep_tma_kernel.  Every wait is bounded; a wait
+// that runs out raises a block flag that ends every other wait of the block, and
+// the kernel leaves with EV_ERROR after the copies still in flight have landed
+// (again bounded).
 constexpr int kTmaConsumers = 256;                    // 8 warps, two groups of 4
 constexpr int kTmaGroup = kTmaConsumers / 2;
 constexpr int kTmaThreads = kTmaConsumers + 32;       // + one producer warp
