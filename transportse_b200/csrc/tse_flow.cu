@@ -34,10 +34,14 @@ struct Walk {
 };
 // The length whose waves of resident blocks take the fewest steps in all, one
 // more a walk for its start (a last wave that is nearly empty costs a full one).
-static Walk walk_of(const TseGrid& g, int out_lanes, int blocks_per_sm) {
+static bool walk_of(const TseGrid& g, int out_lanes, int blocks_per_sm, Walk& w) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+        return false;
     const long long plane = (long long)g.ny * g.nz;
-    const long long warps = (plane + out_lanes - 1) / out_lanes, slots = 148LL * blocks_per_sm;
-    Walk w = {1, (unsigned)((warps + kWalkWarps - 1) / kWalkWarps), 0};
+    const long long warps = (plane + out_lanes - 1) / out_lanes, slots = (long long)sms * blocks_per_sm;
+    w = {1, (unsigned)((warps + kWalkWarps - 1) / kWalkWarps), 0};
     long long best = 0;
     for (int s = kWalkMax; s >= 1; --s) {
         const long long blocks = (long long)w.tiles * ((g.nx + s - 1) / s);
@@ -48,7 +52,7 @@ static Walk walk_of(const TseGrid& g, int out_lanes, int blocks_per_sm) {
             w.blocks = (unsigned)blocks;
         }
     }
-    return w;
+    return true;
 }
 // along x: spacings dx[i0 - 1 .. i0 + steps] and the divisors dx[i] and
 // dx[i] + dx[i + 1] of cells i0 - 1 .. (spacing 1 beside the grid, unused)
@@ -733,7 +737,8 @@ extern "C" int32_t tse_compute_q(const TseGrid* grid, const double* P, const dou
                                                                                  qy, qz, nue, rho_f);
         return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
     }
-    const Walk w = walk_of(*grid, 31, kWalkBlocksQ);
+    Walk w;
+    if (!walk_of(*grid, 31, kWalkBlocksQ, w)) return TSE_ERR_LAUNCH;
     compute_q_kernel<<<w.blocks, kBlock, 0, (cudaStream_t)stream>>>(*grid, w, P, BP, Kx, Ky, Kz, qx, qy, qz,
                                                                   nue, rho_f);
     return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
@@ -753,7 +758,8 @@ extern "C" int32_t tse_flow_error(const TseGrid* grid, const double* P, const do
             *grid, P, Pn, qx, qy, qz, WP, phi, c_f, c_r, rho_f, dt_P, e);
         return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
     }
-    const Walk w = walk_of(*grid, 30, kWalkBlocksE);
+    Walk w;
+    if (!walk_of(*grid, 30, kWalkBlocksE, w)) return TSE_ERR_LAUNCH;
     flow_error_kernel<<<w.blocks, kBlock, 0, (cudaStream_t)stream>>>(*grid, w, P, Pn, qx, qy, qz, WP, phi,
                                                                    c_f, c_r, rho_f, dt_P, e);
     return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
