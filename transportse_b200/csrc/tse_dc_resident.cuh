@@ -387,29 +387,25 @@ static int run_dc_resident(SolveSetup<Form>& S, DcCtl& c, double dt, int cap, in
     // tags count from 1
     if (!cluster && P.nb > 1 && cudaMemsetAsync(base, 0, res_mem_bytes(S.L, kDcResVals), stream) != cudaSuccess)
         return TSE_ERR_LAUNCH;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    if (timing && (cudaEventCreate(&ev0) != cudaSuccess || cudaEventCreate(&ev1) != cudaSuccess ||
-                   cudaEventRecord(ev0, stream) != cudaSuccess))
-        return TSE_ERR_LAUNCH;
     void* args[] = {(void*)&S.F, (void*)&c, (void*)&P, (void*)&w, (void*)&X_out, (void*)&d_status};
-    if (!res_launch(fn, P, threads, cluster, args, stream)) return TSE_ERR_LAUNCH;
-    if (timing) {
-        // the one launch holds the cycles' residuals too
-        int its = 0;
-        float ms = 0.0f;
-        const bool ok = cudaEventRecord(ev1, stream) == cudaSuccess &&
-                        cudaMemcpyAsync(&its, &d_status->num_it, sizeof(int), cudaMemcpyDeviceToHost,
-                                        stream) == cudaSuccess &&
-                        cudaStreamSynchronize(stream) == cudaSuccess &&
-                        cudaEventElapsedTime(&ms, ev0, ev1) == cudaSuccess;
-        cudaEventDestroy(ev0);
-        cudaEventDestroy(ev1);
-        if (!ok) return TSE_ERR_LAUNCH;
-        timing->sweep_launches = 1;
-        timing->sweep_iterations = its;
-        timing->sweep_ms = ms;
-        timing->loop_ms = 0.0;
-    }
+    if (!timing) return res_launch(fn, P, threads, cluster, args, stream) ? TSE_OK : TSE_ERR_LAUNCH;
+    // the one launch holds the cycles' residuals too
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    int its = 0;
+    float ms = 0.0f;
+    const bool ok =
+        cudaEventCreate(&ev0) == cudaSuccess && cudaEventCreate(&ev1) == cudaSuccess &&
+        cudaEventRecord(ev0, stream) == cudaSuccess && res_launch(fn, P, threads, cluster, args, stream) &&
+        cudaEventRecord(ev1, stream) == cudaSuccess &&
+        cudaMemcpyAsync(&its, &d_status->num_it, sizeof(int), cudaMemcpyDeviceToHost, stream) == cudaSuccess &&
+        cudaStreamSynchronize(stream) == cudaSuccess && cudaEventElapsedTime(&ms, ev0, ev1) == cudaSuccess;
+    if (ev0) cudaEventDestroy(ev0);
+    if (ev1) cudaEventDestroy(ev1);
+    if (!ok) return TSE_ERR_LAUNCH;
+    timing->sweep_launches = 1;
+    timing->sweep_iterations = its;
+    timing->sweep_ms = ms;
+    timing->loop_ms = 0.0;
     return TSE_OK;
 }
 
