@@ -17,7 +17,7 @@ def _case(shape, seed):
     return cfg, rng, q, rng.uniform(0.05, 0.3, shape)
 
 
-@pytest.mark.parametrize("shape", [(5, 1, 3), (33, 17, 21), (120, 101, 91)])
+@pytest.mark.parametrize("shape", [(5, 1, 3), (33, 17, 21), (120, 101, 91), (170, 160, 150)])
 @pytest.mark.parametrize("kind", ["all negative", "some negative", "spacings", "tiny", "huge", "underflow"])
 def test_cfl_of_unusual_operands_equals_the_oracle(kind, shape, cuda_device):
     """Every quotient's sign and rounding counts: a maximum of negative

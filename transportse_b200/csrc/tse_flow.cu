@@ -424,19 +424,28 @@ __global__ void l2_partial_kernel(const double* New, const double* Old, long lon
 
 // dt_CFL (tse.py:1241-1246): element f of reshape(|qx|/phi, (ny,nz,nx)) / dx
 // is divided by dx[f % nx]; likewise dy[f % ny]; qz uses dz[k].
-// Bound: DRAM.  |q| / p / d is formed only where it can exceed the warp's
-// maximum so far.  A product tells, with a margin for its rounding, where the
-// maximum, p and d are positive and far from the ends of the exponent range
-// (|q| / p may then round to nothing without reaching the maximum); with any
-// other, and with NaN, the quotient is formed.  Of 160 us at
+// Bound: the divisions, then DRAM.  On large grids |q| / p / d is formed only
+// where it can exceed the warp's maximum so far.  A product tells, with a margin
+// for its rounding, where the maximum, p and d are positive and far from the ends
+// of the exponent range (|q| / p may then round to nothing without reaching the
+// maximum); with any other, and with NaN, the quotient is formed.  Of 160 us at
 // 255 x 256 x 127 the arrays take 41; six divisions and two 64-bit remainders a
-// cell took the rest.  Now 86.
+// cell took the rest.  Now 86.  Below kCflDirect cells a thread has too few cells
+// for a maximum to save much, and the warp's agreement on it costs more (us,
+// direct and not: 23 / 27 at 90^3, 29 / 34 at 128 x 128 x 100, 47 / 50 at 160 x
+// 192 x 101, 56 / 59 at 200 x 190 x 101; 106 / 92-104 at 255 x 256 x 127).
+constexpr long long kCflDirect = 4000000;
+template <bool DIRECT>
 struct CflMax {
-    double m = -HUGE_VAL;   // the warp's
+    double m = -HUGE_VAL;   // the warp's, or the thread's
     __device__ __forceinline__ bool below(double q, double p, double d) const {
         return plain_positive(m) && plain_positive(p) && plain_positive(d) && q * (1.0 + 1e-12) < m * p * d;
     }
     __device__ __forceinline__ void take(double q, double p, double d, bool in) {
+        if (DIRECT) {
+            if (in) m = nmax(m, q / p / d);
+            return;
+        }
         const bool cand = in && !below(q, p, d);
         if (!__any_sync(0xffffffffu, cand)) return;
         double v = cand ? q / p / d : m;
@@ -444,15 +453,17 @@ struct CflMax {
         m = nmax(m, v);
     }
 };
+template <bool DIRECT>
 __global__ void cfl_partial_kernel(TseGrid g, const double* qx, const double* qy, const double* qz,
                                    const double* phi, double* parts) {
     __shared__ double sh[kBlock / 32];
     const long long n = (long long)g.nx * g.ny * g.nz;
     const long long st = (long long)gridDim.x * blockDim.x, f0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    // f % nx, f % ny, f % nz, stepped along
-    const int ax = (int)(st % g.nx), ay = (int)(st % g.ny), az = (int)(st % g.nz);
-    int ix = (int)(f0 % g.nx), iy = (int)(f0 % g.ny), iz = (int)(f0 % g.nz);
-    CflMax a, b, c;
+    // f % nx, f % ny, f % nz, stepped along (st and f0 are below 2^32)
+    const unsigned u = (unsigned)st, v = (unsigned)f0;
+    const int ax = (int)(u % (unsigned)g.nx), ay = (int)(u % (unsigned)g.ny), az = (int)(u % (unsigned)g.nz);
+    int ix = (int)(v % (unsigned)g.nx), iy = (int)(v % (unsigned)g.ny), iz = (int)(v % (unsigned)g.nz);
+    CflMax<DIRECT> a, b, c;
     for (long long w0 = f0 - (threadIdx.x & 31), f = f0; w0 < n; w0 += st, f += st) {
         const bool in = f < n;
         const long long h = in ? f : n - 1;
@@ -788,7 +799,10 @@ extern "C" int32_t tse_dt_cfl(const TseGrid* grid, const double* qx, const doubl
     cudaStream_t s = (cudaStream_t)stream;
     double* parts = (double*)ws;
     const unsigned nb = red_blocks(n);
-    cfl_partial_kernel<<<nb, kBlock, 0, s>>>(*grid, qx, qy, qz, phi, parts);
+    if (n < kCflDirect)
+        cfl_partial_kernel<true><<<nb, kBlock, 0, s>>>(*grid, qx, qy, qz, phi, parts);
+    else
+        cfl_partial_kernel<false><<<nb, kBlock, 0, s>>>(*grid, qx, qy, qz, phi, parts);
     if (cudaGetLastError() != cudaSuccess) return TSE_ERR_LAUNCH;
     static const int ops[3] = {R_MAX, R_MAX, R_MAX};
     return finish(parts, nb, 3, ops, d_out, 2, ws, s);
