@@ -23,10 +23,17 @@ __device__ __forceinline__ void decode(long long t, int ny, int nz, int& i, int&
 // repeat cells of the next one.
 constexpr int kWalkMax = 16;
 // From these grid sizes on; below, a thread a cell keeps the SMs fuller (us,
-// thread a cell against walks: fluxes 31 / 33 at 96^3, 56 / 51 at 112^3, 130 / 105
-// at 160 x 192 x 101; flow error 5.2 / 6.5 at 48^3, 16 / 14 at 80^3, 99 / 75).
+// thread a cell against walks: fluxes 36 / 39 at 96^3, 74 / 57 at 112^3, 156 / 111
+// at 160 x 192 x 101; flow error 5.2 / 6.5 at 48^3, 18.5 / 16.6 at 80^3, 101 / 85).
+// On a plane (ny = 1) a thread a cell skips the y faces that a walk forms all the
+// same: flow error 14.4 / 18.5 at 1000 x 1 x 500, 53 / 60 at 2000 x 1 x 1000.
 constexpr long long kWalkCellsQ = 1200000, kWalkCellsE = 400000;
-constexpr int kWalkBlocksQ = 4, kWalkBlocksE = 4;   // resident on a SM
+// Blocks resident on a SM.  Flow error: 3 below kWalkCellsE4 cells, where another
+// block's shorter walks start over more often, else 4 (us with 3 / 4: 22.5 / 24.9
+// at 90^3, 47 / 49 at 128 x 128 x 100, 62 / 58 at 128^3, 231 / 221 at 255 x 256 x
+// 127, launched alone).
+constexpr int kWalkBlocksQ = 4;
+constexpr long long kWalkCellsE4 = 2000000;
 constexpr int kWalkWarps = kBlock / 32;
 struct Walk {
     int steps;                // cells of a walk
@@ -148,8 +155,7 @@ __device__ __forceinline__ double mobility(double dsum, const Perm& a, const Per
 }
 
 // 255 x 256 x 127 (B200): 418 us with a thread a cell and the operator's
-// divisions, 265 now (10 arrays, 101 us); a tenth more with 2 or 3 blocks a SM or
-// with 5.  Bound: 15 reciprocals and 23 quotients a cell and the loads' latency
+// divisions, 286 now (10 arrays, 101 us); 302 with 3 blocks a SM, 318 with 5.  Bound: 15 reciprocals and 23 quotients a cell and the loads' latency
 // (FP64 pipe 42 % busy, 28 warps a SM, DRAM 30 %).
 __global__ void __launch_bounds__(kBlock, kWalkBlocksQ)
     compute_q_kernel(TseGrid g, Walk w, const double* P, const double* BP, const double* Kx, const double* Ky,
@@ -271,10 +277,10 @@ __device__ __forceinline__ double harm_of(double dsum, double a1, double a2) {
 }
 
 // A face's mean density is the same bits from either side.  255 x 256 x 127
-// (B200): 305 us before, 190 now (11 arrays, 112 us); a tenth more with 2 blocks a SM
-// or with 4.  Bound: 7 reciprocals and 18 quotients a cell and the loads'
+// (B200): 305 us with a thread a cell, 221 now (11 arrays, 112 us).  Bound: 7 reciprocals and 18 quotients a cell and the loads'
 // latency (FP64 pipe 41 % busy, 21 warps a SM, DRAM 45 %).
-__global__ void __launch_bounds__(kBlock, kWalkBlocksE)
+template <int BLOCKS>
+__global__ void __launch_bounds__(kBlock, BLOCKS)
     flow_error_kernel(TseGrid g, Walk w, const double* P, const double* Pn, const double* qx, const double* qy,
                       const double* qz, const double* WP, const double* phi, const double* c_f,
                       const double* c_r, const double* rho, double dt_P, double* e) {
@@ -764,15 +770,16 @@ extern "C" int32_t tse_flow_error(const TseGrid* grid, const double* P, const do
         return TSE_ERR_ARG;
     const long long n = (long long)grid->nx * grid->ny * grid->nz;
     if (n <= 0) return TSE_ERR_ARG;
-    if (n < kWalkCellsE) {
+    if (n < kWalkCellsE || grid->ny == 1) {
         flow_error_cells_kernel<<<grid_for(n), kBlock, 0, (cudaStream_t)stream>>>(
             *grid, P, Pn, qx, qy, qz, WP, phi, c_f, c_r, rho_f, dt_P, e);
         return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
     }
+    const bool four = n >= kWalkCellsE4;
     Walk w;
-    if (!walk_of(*grid, 30, kWalkBlocksE, w)) return TSE_ERR_LAUNCH;
-    flow_error_kernel<<<w.blocks, kBlock, 0, (cudaStream_t)stream>>>(*grid, w, P, Pn, qx, qy, qz, WP, phi,
-                                                                   c_f, c_r, rho_f, dt_P, e);
+    if (!walk_of(*grid, 30, four ? 4 : 3, w)) return TSE_ERR_LAUNCH;
+    (four ? flow_error_kernel<4> : flow_error_kernel<3>)<<<w.blocks, kBlock, 0, (cudaStream_t)stream>>>(
+        *grid, w, P, Pn, qx, qy, qz, WP, phi, c_f, c_r, rho_f, dt_P, e);
     return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
 }
 
