@@ -459,12 +459,9 @@ __device__ __forceinline__ double qdiv(double a, double2 b) {
     const double r = __fma_rn(__fma_rn(-b.x, q, a), b.y, q);
     return (__double2hiint(q) & 0x7ff00000) == 0x7ff00000 ? q : r;   // inf, NaN
 }
-// A divisor and its reciprocal.  An infinite one (a steady state's dt, a product
-// of spacings) goes along as {0, 0}: the correction is then 0, where -inf 0 + a
-// would be NaN, and the quotient a 0.
-__device__ __forceinline__ double2 with_reciprocal(double b) {
-    return fabs(b) < HUGE_VAL ? make_double2(b, 1.0 / b) : make_double2(b == b ? 0.0 : b, b == b ? 0.0 : b);
-}
+// An infinite divisor (a steady state's dt, a product of spacings) goes along as
+// {0, 0}: the correction is then 0, where -inf 0 + a would be NaN, and the
+// quotient a 0.
 // |v| far from both ends of the exponent range (and not 0, inf or NaN)
 __device__ __forceinline__ bool mid_range(double v) {
     const unsigned e = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu;
@@ -499,9 +496,11 @@ __global__ void axis_tables_kernel(TseGrid g, double2* tab) {
         b[3] = d[i + 1] + dd;
     }
     if (i > 0) b[2] = (0.5 * (d[i - 1] + dd)) * dd;
-    // the first and the last divisor are spacings too
-    for (int q = 0; q < kTabPairs; ++q)
-        t[q * st] = q == 1 || q == 2 ? with_reciprocal(b[q]) : make_double2(b[q], 1.0 / b[q]);
+    // an infinite product as {0, 0}, see qdiv; the others are spacings too
+    for (int q = 0; q < kTabPairs; ++q) {
+        const double r = 1.0 / b[q];
+        t[q * st] = make_double2(r == 0.0 && (q == 1 || q == 2) ? 0.0 : b[q], r);
+    }
 }
 static size_t axis_table_bytes(const Layout& L) {
     return align256((size_t)(L.nx + L.ny + L.nz) * kTabPairs * sizeof(double2));
@@ -630,12 +629,14 @@ struct HeatFast {
 // blocks a SM help as long as registers last (species 630 us with 4 blocks, heat
 // 858 with 5), loads gathered ahead of the arithmetic cost more registers than
 // they hide (species 640 and more).
-template <class Kind, bool LEAN>
+// STEADY: a.dt is infinite (an instance of its own costs the others nothing; a
+// test of dt in the kernel 1 % of a call).
+template <class Kind, bool LEAN, bool STEADY>
 __global__ void __launch_bounds__(kBlock, Kind::kBlocks)
     assemble_fast_kernel(TseGrid g, typename Kind::Args a, TransportForm F, uint8_t* mask0, uint8_t* mask1,
                          Layout L, const double2* __restrict__ tab, DcFuse fz) {
     __shared__ double sh[kBlock / 32];
-    const double2 dt = with_reciprocal(a.dt);
+    const double2 dt = STEADY ? make_double2(0.0, 0.0) : make_double2(a.dt, 1.0 / a.dt);
     const double omega = F.omega;
     const long long N = F.Ncal;
     const int ts = L.nx + L.ny + L.nz;
@@ -834,12 +835,10 @@ static int assemble_fast(const TseGrid* grid, const typename Kind::Args* a, Tran
     TransportForm F = S.F;
     F.useY = a->omega != 1.0;
     F.useEX = a->imblflo != 0;
-    if (S.lean)
-        assemble_fast_kernel<Kind, true><<<(unsigned)nb, kBlock, 0, stream>>>(*grid, *a, F, S.mask[0], S.mask[1],
-                                                                               S.L, tab, fz);
-    else
-        assemble_fast_kernel<Kind, false><<<(unsigned)nb, kBlock, 0, stream>>>(*grid, *a, F, S.mask[0],
-                                                                                S.mask[1], S.L, tab, fz);
+    const bool steady = std::isinf(a->dt);
+    auto kernel = S.lean ? (steady ? assemble_fast_kernel<Kind, true, true> : assemble_fast_kernel<Kind, true, false>)
+                         : (steady ? assemble_fast_kernel<Kind, false, true> : assemble_fast_kernel<Kind, false, false>);
+    kernel<<<(unsigned)nb, kBlock, 0, stream>>>(*grid, *a, F, S.mask[0], S.mask[1], S.L, tab, fz);
     *nparts = (int)nb;
     return cudaGetLastError() == cudaSuccess ? TSE_OK : TSE_ERR_LAUNCH;
 }
