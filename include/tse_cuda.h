@@ -73,7 +73,8 @@ typedef struct TseSolveStatus {
     double ev_dt[8];
     double ev_diff[8];
     int32_t cycles;    /* mixed-precision forms: FP64 residual evaluations */
-    int32_t sweep;     /* FP64 forms: the kernel that ran, TSE_SWEEP_*; else 0 */
+    int32_t sweep;     /* FP64 forms: the kernel that ran, TSE_SWEEP_* (the others
+                          leave it) */
 } TseSolveStatus;
 enum { TSE_SWEEP_PLAIN = 1, TSE_SWEEP_STAGED = 2, TSE_SWEEP_RESIDENT = 3 };
 

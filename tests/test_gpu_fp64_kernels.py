@@ -60,15 +60,3 @@ def test_the_chosen_kernel_runs_and_all_agree(shape, pressure, species, cuda_dev
         for a, b in zip(out[0], other):
             for x, y in zip(a, b):
                 assert numpy.array_equal(x, y, equal_nan=True)
-
-
-def test_a_mixed_precision_solve_reports_no_fp64_kernel(cuda_device):
-    from transportse_b200 import workloads
-    cfg = workloads.base_config("dc", 12, 11, 10, 1.0, 1.0, 1.0)
-    one = numpy.ones((12, 11, 10))
-    args = (4.5e-10 * one, 1e-3 * one, 1e3 * one, 0.2 * one, 1e-12 * one, 1e-12 * one, 1e-12 * one, one, one, one)
-    for precision, sweep in (("fp32dc", 0), ("fp64", RESIDENT)):
-        m = model_for(cfg, cuda_device, precision)
-        m.status.fill_(7)
-        m.compute_P(1e5 * one, *args, 3600.0, 0 * one, 0 * one, P_conv=1e-6)
-        assert m.last_status.sweep == sweep

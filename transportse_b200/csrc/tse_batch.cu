@@ -245,7 +245,6 @@ __device__ void cluster_dc_solve(cg::cluster_group& cl, const BatchItem<Form>& i
         st->error = TSE_STATUS_OK;
         st->n_events = nev < 8 ? nev : 8;
         st->cycles = cycles;
-        st->sweep = 0;
     }
     // compact colour arrays -> natural (nx, ny, nz); the last barrier above
     // made every x visible

@@ -659,7 +659,6 @@ __global__ void dc_status_kernel(const DcState* st, TseSolveStatus* s) {
         s->ev_diff[q] = st->ev_diff[q];
     }
     s->cycles = st->cycles;
-    s->sweep = 0;
 }
 
 // ------------------------------------------------------------------ host

@@ -318,7 +318,6 @@ __global__ void __launch_bounds__(NT, 1)
         s->error = failed ? TSE_STATUS_BARRIER_TIMEOUT : TSE_STATUS_OK;
         s->n_events = nev < 8 ? nev : 8;
         s->cycles = cycles;
-        s->sweep = 0;
     }
 }
 
