@@ -46,7 +46,9 @@ constexpr int kMaxBlocks = 16384;
 constexpr int kPlainBlock = 768;
 // From this many cells of a colour on the staged sweep (tse_rbsolve_tma.cuh) is
 // the faster one, below this one (staged / plain: 72^3 19.3 / 12.9, 100^3 30.2 /
-// 27.6, 110^3 35.8 / 33.4, 128 x 128 x 127 47.1 / 46.4, 192 x 160 x 101 65.1 / 74.4).
+// 27.6, 110^3 35.8 / 33.4, 128 x 128 x 127 47.1 / 46.4, 192 x 160 x 101 65.1 / 74.4;
+// 1300 x 1 x 1300 54.9 / 40.7).  A pressure solve of fewer than 50 iterations, which
+// all check, is 2-5 % slower plain from 0.7 M cells on.
 constexpr long long kStagedMinNc = 1000000;
 
 // `sweep` as the entry points take it: 1 plain, 2 staged, else by size
