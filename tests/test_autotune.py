@@ -79,3 +79,20 @@ def test_the_ensemble_tuner_is_not_misled_by_a_first_run(monkeypatch):
     monkeypatch.setattr(ensemble, "Ensemble", Runs)
     best = ensemble.autotune([None], batched=True, clusters=(0,), cycles=(512, 256, 128))
     assert best["dc_cycle"] == 512 and [t["rate"] for t in best["trials"]] == [73.0, 70.0, 69.0]
+
+
+@pytest.mark.parametrize("rates,chosen", [({128: 75.9, 256: 81.5, 512: 81.4}, 512), ({128: 82.0, 256: 70.0, 512: 60.0}, 128),
+                                          ({128: 80.0, 256: 80.4, 512: 78.0}, 256)])
+def test_the_ensemble_tuner_takes_the_longest_cycle_of_equals(rates, chosen, monkeypatch):
+    """Rates within a sample's spread do not decide."""
+    from transportse_b200 import ensemble
+
+    class Runs:
+        def __init__(self, configs, device=None, precision=None, **p):
+            self.p = p
+
+        def run(self, steps, keep=()):
+            return [], {"stepping_cell_updates_per_s": rates[self.p["dc_cycle"]], "cell_updates_per_s": 1.0}
+
+    monkeypatch.setattr(ensemble, "Ensemble", Runs)
+    assert ensemble.autotune([None], batched=True, clusters=(0,), cycles=(128, 256, 512))["dc_cycle"] == chosen

@@ -165,6 +165,10 @@ def run_model(config, steps, device, precision, max_blocks, dc_cycle=None, keep=
     return step_model(sim, steps, keep, gate)
 
 
+# rates of a tuning sample closer than this are alike
+TUNE_SPREAD = 0.02
+
+
 def autotune(configs, device=None, precision="fp32dc", steps=1, concurrency=(2, 4, 8),
              cycles=(128,), cluster_cells=(0,), batched=False, clusters=(8, 16)):
     """Pick the launch shape that gives the highest cell-update rate on a
@@ -173,7 +177,8 @@ def autotune(configs, device=None, precision="fp32dc", steps=1, concurrency=(2, 
     correction-cycle length; batched, the cluster size (CTAs per model) and
     cycle length.  Returns the best parameter set with its "rate" and all
     "trials"; the sample runs from the models' initial state each time, twice
-    per set, and the better run counts."""
+    per set, and the better run counts; of sets within TUNE_SPREAD of the best
+    rate the one with the longest cycle is taken."""
     space = []
     if batched:
         for c in clusters:
@@ -186,7 +191,6 @@ def autotune(configs, device=None, precision="fp32dc", steps=1, concurrency=(2, 
                     space.append({"batched": False, "concurrency": k, "cluster_cells": cc,
                                   "dc_cycle": cyc})
     trials = []
-    best = None
     for p in space:
         # the better of two runs: the first one in a process allocates inside
         # its steps (34 against 70 G cell-updates/s on 16 models), and a host
@@ -197,8 +201,12 @@ def autotune(configs, device=None, precision="fp32dc", steps=1, concurrency=(2, 
             # the stepping phase's rate where set-up is apart (it dominates short samples)
             rate = max(rate, st["stepping_cell_updates_per_s"] or st["cell_updates_per_s"])
         trials.append(dict(p, rate=rate))
-        if best is None or trials[-1]["rate"] > best["rate"]:
-            best = dict(trials[-1])
+    # a sample's rates repeat to a per cent or two; of sets that close to the best
+    # the longest cycle, which launches least (256 and 512 iterations: 81.5 and
+    # 81.4 G/s on 16 models, 114 and 117 on 512)
+    top = max(t["rate"] for t in trials)
+    best = dict(max((t for t in trials if t["rate"] >= (1.0 - TUNE_SPREAD) * top),
+                    key=lambda t: (t["dc_cycle"], t["rate"])))
     best["trials"] = trials
     return best
 
