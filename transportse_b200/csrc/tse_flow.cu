@@ -436,7 +436,7 @@ __global__ void l2_partial_kernel(const double* New, const double* Old, long lon
 // of the exponent range (|q| / p may then round to nothing without reaching the
 // maximum); with any other, and with NaN, the quotient is formed.  Of 160 us at
 // 255 x 256 x 127 the arrays take 41; six divisions and two 64-bit remainders a
-// cell took the rest.  Now 86.  Below kCflDirect cells a thread has too few cells
+// cell took the rest.  Now 92.  Below kCflDirect cells a thread has too few cells
 // for a maximum to save much, and the warp's agreement on it costs more (us,
 // direct and not: 23 / 27 at 90^3, 29 / 34 at 128 x 128 x 100, 47 / 50 at 160 x
 // 192 x 101, 56 / 59 at 200 x 190 x 101; 106 / 92-104 at 255 x 256 x 127).
